@@ -73,7 +73,8 @@ def work_by_kernel(arrays, counters: np.ndarray):
     steps, rhs, jac, fact, solve = c[0], c[1], c[2], c[3], c[4]
     w_rhs = rhs * f_rhs + jac * ((n - 1) * f_cached + f_rhs)
     w_adv = fact * (2.0 / 3.0 * n ** 3 + n * n) + solve * 2.0 * n * n + jac * n * n + steps * VEC_FLOPS_PER_N * n
-    return {"rhs": w_rhs, "advance": w_adv, "plain": w_rhs + w_adv, "persistent": w_rhs + w_adv}
+    return {"rhs": w_rhs, "advance": w_adv, "plain": w_rhs + w_adv, "persistent": w_rhs + w_adv,
+            "group": w_rhs + w_adv}
 
 
 def fp64_peak_tflops(device) -> float:
@@ -129,7 +130,7 @@ def kernel_roofline(args, ktimes, counters, arrays, fp64_peak, hbm, hbm_src):
             "peak_source": "measured live in this run: cuBLAS DGEMM 8192^3, CUDA events",
             "hbm_view": {"algorithmic_bytes_per_launch": step_bytes, "achieved_gbs": step_bytes / avg_s / 1e9,
                          "peak_gbs": hbm, "peak_source": hbm_src},
-            "note": "latency-bound BDF solver kernel; traffic is its cell-record round trips"}
+            "note": "latency-bound BDF solver kernel"}
 
 
 def tuning_report(ctx, lsg):
@@ -137,9 +138,9 @@ def tuning_report(ctx, lsg):
     if t is None:
         return None
     tile, width, rates = t
-    names = {lsg.LSG_TILE_LANE: f"round scheme, {width} lanes per cell", lsg.LSG_TILE_WARP: "plain warp kernel",
+    names = {lsg.LSG_TILE_LANE: f"batched form, {width} lanes per cell", lsg.LSG_TILE_WARP: "plain warp kernel",
              lsg.LSG_TILE_PERSISTENT: "persistent lane kernel",
-             lsg.LSG_TILE_GROUP: f"fused lane-group kernel, {width} blocks per SM",
+             lsg.LSG_TILE_GROUP: "resident kernel, " + ("32 lanes" if width == 2 else "16 lanes") + " per cell",
              lsg.LSG_TILE_BLOCK: "block per cell, " + ("tensor-core inverse" if width else "FP64 LU factors")}
     return {"chosen": names.get(tile, str(tile)), "sample_cells_per_s": {k: round(v) for k, v in rates.items() if v}}
 

@@ -47,13 +47,14 @@ extern "C" {
 #define LSG_PRECISION_MIXED 1  /* FP64 rates/residual/error control, FP32 factorisation + FP64 refinement */
 
 /* work decomposition (lsg_options.tile) */
-#define LSG_TILE_AUTO 0        /* FP64 -> warp per cell; MIXED -> lane per cell (up to 31 species) */
+#define LSG_TILE_AUTO 0        /* FP64 -> warp per cell; MIXED -> the batched form (up to 31 species) */
 #define LSG_TILE_WARP 1        /* one warp per cell, the reference's operation order (FP64 only) */
-#define LSG_TILE_LANE 2        /* one thread per cell, rounds of RHS / solver / factor kernels over the live cells */
+#define LSG_TILE_LANE 2        /* the batched form: cells resident in shared memory from start to finish, many to a
+                                  block, or (few cells a block, analytic Jacobian) rounds of RHS / solver kernels over
+                                  the live cells; the same results either way */
 #define LSG_TILE_PERSISTENT 3  /* one thread per cell, one persistent kernel + device work queue */
 #define LSG_TILE_BLOCK 4       /* one thread block per cell (any size up to 511 species) */
-#define LSG_TILE_GROUP 5       /* one lane group (16 or 32 lanes) per cell from start to finish, the RHS evaluated
-                                  by the group inside the solver kernel, persistent grid (up to 31 species) */
+#define LSG_TILE_GROUP 5       /* the batched form's resident kernel, called asynchronously (up to 31 species) */
 /* Mechanisms of 32 to 511 species always run one thread block per cell (the
  * tile is ignored).  The block form factorises in FP64 with LSG_PRECISION_FP64.
  * With LSG_PRECISION_MIXED it inverts G = I - h r0 J on the tensor cores in
@@ -104,8 +105,8 @@ typedef struct lsg_options {
  * it by forward differences, one RHS evaluation per column
  * (KernelDense.hpp:111-193).  LSG_JACOBIAN_ANALYTIC differentiates the rate
  * expressions for the species columns (lsg_jacobian_device) and keeps the
- * temperature column a forward difference; it is used by the lane-per-cell
- * round scheme (LSG_TILE_LANE) of the constant-pressure reactor, the other
+ * temperature column a forward difference; it is used by the
+ * batched form (LSG_TILE_LANE) of the constant-pressure reactor, the other
  * forms and the constant-volume reactor keep the differences.  It changes the
  * Newton iterates (not their fixed point), so step sequences can differ from
  * the reference's at O(rtol). */
@@ -169,7 +170,7 @@ int lsg_reaction_step_device(lsg_ctx* ctx, int ncells, int nspecies, double* Y_d
  * captured once into a CUDA graph on the context's stream and replayed;
  * the context keeps the graph and replays it while every argument stays the
  * same (a changed argument or lsg_ctx_set_options captures anew).  The form
- * whose rounds wait on the host (LSG_TILE_LANE, or the autotuner's choice of
+ * whose calls wait for the step (LSG_TILE_LANE, or the autotuner's choice of
  * it) runs the steps one by one instead.  graph_used (optional) is set to 1
  * when the graph ran.  Ordered after the work already on `stream` and before
  * the work enqueued on it afterwards; asynchronous.  No counterpart in the
@@ -252,20 +253,20 @@ long long lsg_ctx_launches(const lsg_ctx* ctx);
 /* Device time per kernel kind, from CUDA events recorded on the launching
  * stream when lsg_options.kernel_timing is set (diagnostics; no counterpart in
  * the reference).  Kinds: 0 RHS, 1 solver advance, 2 compaction, 3 round
- * initialisation (lane-per-cell form), 4 plain warp kernel, 5 persistent lane
- * kernel, 6 block-per-cell kernel (large mechanisms), 7 fused lane-group
- * kernel.  ms[k] total milliseconds, launches[k] timed launches; reset != 0
+ * initialisation (the batched form's rounds), 4 plain warp kernel, 5 persistent lane
+ * kernel, 6 block-per-cell kernel (large mechanisms), 7 the batched form's
+ * resident kernel.  ms[k] total milliseconds, launches[k] timed launches; reset != 0
  * clears the totals after reading.  Waits for the last timed kernel. */
 #define LSG_NKERNEL_KINDS 8
 int lsg_ctx_kernel_times(lsg_ctx* ctx, double* ms, long long* launches, int nkinds, int reset);
 
 /* Result of the autotuner (lsg_options.autotune; no counterpart in the
  * reference): the chosen tile and its variant (lanes per cell, 16 or 32, for
- * the round scheme; blocks per SM, 4 or 2, for the fused lane-group kernel; 0
- * otherwise) and the measured cells/s of the candidates, in the order round
- * scheme 16 lanes, round scheme 32 lanes, plain warp kernel, persistent lane
- * kernel, fused lane-group kernel at 4 and at 2 blocks per SM (0 for a
- * candidate not tried).  For mechanisms above 31 species with
+ * the batched form; 4: 16 lanes where the components fit, 2: 32 lanes, for its
+ * resident kernel called as LSG_TILE_GROUP; 0 otherwise) and the measured
+ * cells/s of the candidates, in the order batched form 16 lanes, batched form
+ * 32 lanes, plain warp kernel, persistent lane kernel, resident kernel variants
+ * 4 and 2 (0 for a candidate not tried).  For mechanisms above 31 species with
  * LSG_PRECISION_MIXED the candidates are the block form with FP64 LU factors
  * (rates[0]) and with the tensor-core inverse (rates[1]), timed on one wave of
  * the FP64 form's blocks (at least 256 cells); tile is then LSG_TILE_BLOCK and

@@ -58,7 +58,7 @@ struct lsg_ctx {
   long bws_blocks = 0;
   long tc_blocks = 0;           // blocks of the tensor-core (mixed-precision) block kernel
   int* bqueue = nullptr;
-  int* gqueue = nullptr;        // cell queue of the fused lane-group form
+  int* gqueue = nullptr;        // cell queue of the resident form
   KernelTimer timer;          // per-kernel device time (lsg_options.kernel_timing)
   // autotuner (lsg_options.autotune)
   bool tuned = false;
@@ -374,15 +374,15 @@ int tune_sample(lsg_ctx* c, const StepArgs& a, cudaStream_t s, long m, StepArgs*
 }
 
 // Autotuner: times the candidate forms on (a copy of) the first cells of the
-// call (up to 262,144) and keeps the fastest for tile LSG_TILE_AUTO.  Candidates: round scheme
-// with 16-lane groups (two cells per warp, up to 16 equations) and with 32-lane
-// groups, the plain warp kernel (FP64 only) and the persistent lane kernel.
+// call (up to 262,144) and keeps the fastest for tile LSG_TILE_AUTO.  Candidates: the batched form
+// with 16 lanes a cell (two cells per warp, up to 16 equations) and with 32, the plain warp kernel
+// (FP64 only), the persistent lane kernel and the resident form called directly.
 int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
   const MechLayout& L = c->mech->host.layout;
   const int nc = L.nc, n = nc + 1;
   (void)nc;
-  // The round scheme needs many cells to hide its latency: a small sample would
-  // under-rate it, so the sample is up to 262,144 cells (a one-time cost).
+  // The forms need many cells to hide their latency: a small sample would
+  // under-rate them, so the sample is up to 262,144 cells (a one-time cost).
   const long m = a.ncells < 262144 ? a.ncells : 262144;
   StepArgs t;
   double *pristine = nullptr, *work = nullptr;
@@ -501,12 +501,40 @@ int launch_step(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
   return launch_tile(c, a, s, tile);
 }
 
+// The resident form's kernel (lsg_team.cuh), enqueued.
+int launch_resident(lsg_ctx* c, const StepArgs& a, const StepOptions& so, int width, cudaStream_t s) {
+  if (!c->gqueue && cudaMalloc(&c->gqueue, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return LSG_ERR_NOMEM; }
+  if (c->timer.used >= KernelTimer::kPairs) {
+    cudaStreamSynchronize(s);
+    c->timer.collect();
+  }
+  c->timer.begin(KT_GROUP, s);
+  const cudaError_t e = launch_group(c->mech->host.layout, c->mech->d_buf, so, a,
+                                     c->opt.precision == LSG_PRECISION_FP64, width, c->gqueue, c->sm_count, s);
+  c->timer.end(s);
+  if (e == cudaErrorInvalidValue) { cudaGetLastError(); return LSG_ERR_UNSUPPORTED; }
+  if (e != cudaSuccess) return LSG_ERR_CUDA;
+  c->launches += 1;
+  return LSG_OK;
+}
+
 int launch_tile(lsg_ctx* c, const StepArgs& a, cudaStream_t s, int tile) {
   const MechLayout& L = c->mech->host.layout;
   const StepOptions so = to_step_options(c->opt);
   if (L.nc + 1 > 32 || tile == LSG_TILE_BLOCK) return launch_large(c, a, s);
+  if (tile == LSG_TILE_GROUP && !resident_fits(L)) tile = LSG_TILE_LANE;   // the same solver in rounds
   if (tile == LSG_TILE_LANE) {
     const bool lu64 = c->opt.precision == LSG_PRECISION_FP64;
+    const int width = c->tuned ? c->tuned_w : 0;
+    if (!sm_count(c)) return LSG_ERR_CUDA;
+    if (resident_applies(L, so, a.ncells, width, c->sm_count)) {
+      const int r = launch_resident(c, a, so, width, s);
+      if (r != LSG_OK) return r;
+      // as with the round scheme, the call returns when the step is done
+      if (cudaStreamSynchronize(s) != cudaSuccess) return LSG_ERR_CUDA;
+      c->timer.collect();
+      return LSG_OK;
+    }
     const int r = ensure_rounds(c, a.ncells, lu64);
     if (r != LSG_OK) return r;
     const long max_rounds = 4L * (long)c->opt.max_steps * (L.nc + 9) + 64;
@@ -517,21 +545,9 @@ int launch_tile(lsg_ctx* c, const StepArgs& a, cudaStream_t s, int tile) {
   }
   if (tile == LSG_TILE_GROUP) {
     if (L.nc + 1 > 32) return LSG_ERR_UNSUPPORTED;
-    if (!c->gqueue && cudaMalloc(&c->gqueue, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return LSG_ERR_NOMEM; }
     if (!sm_count(c)) return LSG_ERR_CUDA;
-    if (c->timer.used >= KernelTimer::kPairs) {
-      cudaStreamSynchronize(s);
-      c->timer.collect();
-    }
-    const int mb = (c->tuned && c->tuned_w == 2) ? 2 : 4;   // the autotuner's occupancy variant, else 4 blocks/SM
-    c->timer.begin(KT_GROUP, s);
-    const cudaError_t e = launch_group(L, c->mech->d_buf, so, a, c->opt.precision == LSG_PRECISION_FP64,
-                                       mb == 2 ? 2 : 4, c->gqueue, c->d_err, c->sm_count, s);
-    c->timer.end(s);
-    if (e == cudaErrorInvalidValue) { cudaGetLastError(); return LSG_ERR_UNSUPPORTED; }
-    if (e != cudaSuccess) return LSG_ERR_CUDA;
-    c->launches += 1;
-    return LSG_OK;
+    // the autotuner's variant 2: a warp a cell; else 16 lanes where the components fit
+    return launch_resident(c, a, so, (c->tuned && c->tuned_w == 2) ? 32 : 0, s);
   }
   if (tile == LSG_TILE_WARP) {
     if (L.nc + 1 > 32) return LSG_ERR_UNSUPPORTED;
@@ -873,7 +889,7 @@ int lsg_reaction_step_cv_device(lsg_ctx* c, int ncells, int nspecies, double* Y,
 }
 
 // A sequence of device-resident steps, captured once into a CUDA graph and replayed while the arguments
-// stay the same.  Forms whose step waits on the host (the round scheme) run the steps one by one.
+// stay the same.  The batched form, whose calls wait for the step, runs the steps one by one.
 int lsg_reaction_step_sequence_device(lsg_ctx* c, int nsteps, int ncells, int nspecies, double* Y, long ld,
                                       double* T, double p, double t0, double dt, double* Q, int* status,
                                       int* graph_used, void* stream) {
@@ -894,7 +910,8 @@ int lsg_reaction_step_sequence_device(lsg_ctx* c, int nsteps, int ncells, int ns
   }
   int tile = (c->tuned && c->opt.tile == LSG_TILE_AUTO) ? c->tuned_tile : resolve_tile(c->opt);
   if (L.nc + 1 > 32) tile = LSG_TILE_BLOCK;
-  if (tile == LSG_TILE_LANE) {   // host-synchronised rounds: no graph
+  if (tile == LSG_TILE_GROUP && !resident_fits(L)) tile = LSG_TILE_LANE;
+  if (tile == LSG_TILE_LANE) {   // the call waits for each step: no graph
     for (int k = 0; k < nsteps; ++k) {
       a.t0 = t0 + k * dt;
       const int r = launch_tile(c, a, s, tile);

@@ -161,10 +161,12 @@ cudaError_t launch_rounds(const RoundsPlan& P, const MechLayout& L, const unsign
 cudaError_t launch_rhs_warp(const MechLayout& L, const unsigned char* mech_gmem, long ncells, const double* y,
                             double* dy, long ld, double p, int energy, double* qr, int* err, cudaStream_t stream);
 
-// Fused lane-group form (lsg_rounds.cu): one lane group per cell from start to finish, RHS in-kernel;
-// min_blocks 4 or 2 blocks per SM (128 or 255 registers a thread); queue: one int
+// Resident form (lsg_team.cuh): a block's cells stay in shared memory from start to finish; width lanes a cell (16,
+// 32 or 0: by the number of components); queue: one int
 cudaError_t launch_group(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o, const StepArgs& a,
-                         bool lu64, int min_blocks, int* queue, int* err, int sm_count, cudaStream_t stream);
+                         bool lu64, int width, int* queue, int sm_count, cudaStream_t stream);
+bool resident_fits(const MechLayout& L);   // a block's shared memory holds at least one warp's cells
+bool resident_applies(const MechLayout& L, const StepOptions& o, long ncells, int width, int sm_count);
 
 // Jacobians with analytic species columns (lsg_rounds.cu), up to 31 species; J [ncells][n][n] row-major
 cudaError_t launch_jacobian(const MechLayout& L, const unsigned char* mech_gmem, long ncells, const double* y, long ld,

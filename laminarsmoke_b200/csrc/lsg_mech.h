@@ -50,7 +50,19 @@ struct MechLayout {
   int tb_ptr, tb_sp;                                         // third body CSR (by slot)
   int fo_type, fo_single, fo_ptr, fo_sp;                     // fall-off (by slot)
   int fo_cabr;                                               // 1: chemically activated bimolecular (by slot)
+  // ---- the reactions once more for the small-mechanism kernels (up to 31 species)
+  int rx_dat;                                                // double [nr][4]: lnA, beta, E/R, dnu
+  int fg_ent;                                                // double [nnz][2]: signed coefficient, reaction (an int)
+  int fg_exact;                                              // every coefficient is +-1 or +-2
+  int rx_pack;                                               // int [nr][4]: species bytes, kRx* flags, tb slot, fo slot
+  int rx_order;                                              // int [nr]: fall-off first, special forms, the rest
+  int fg_ptr;                                                // per species CSR of fg_ent: reaction order, reactants first
 };
+
+// Packed reaction (rx_pack): up to two reactants and two products with coefficient one, or one with two (named
+// twice), an absent second species named nc (concentration 1, g 0), so that the kernels multiply and add without
+// loops or branches.  kRxSpecial: none of that holds, the general tables apply.
+enum : int { kRxSpecial = 1, kRxReversible = 2, kRxTwice = 4, kRxNegative = 8 };
 
 // Fitted transport properties (the packed blob's tr_* arrays), flattened into
 // a table of their own: [double region][int region], offsets in elements.

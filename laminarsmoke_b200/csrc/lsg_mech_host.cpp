@@ -131,6 +131,105 @@ static bool build_transport(const Blob& b, int nc, HostMech& out, std::string& e
   return true;
 }
 
+namespace {
+// The packed reaction table and the reaction-ordered formation-rate lists (mech.h rx_*, fg_*), for mechanisms
+// of up to 31 species; larger ones get empty tables.
+void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::vector<int>& tb_slot,
+                    const std::vector<int>& fo_slot, const std::vector<int>& plog_slot,
+                    const std::vector<int>& cheb_slot, Builder& B, MechLayout& L) {
+  const int nc = L.nc, nr = L.nr;
+  std::vector<double> dat(4, 0.), ent(2, 0.);
+  std::vector<int> pack(4, 0), order(1, 0), ptr(1, 0);
+  L.fg_exact = 1;
+  if (nc <= 31) {
+    const auto& rp = b.I("reac_ptr");
+    const auto& rs = b.I("reac_species");
+    const auto& rn = b.F("reac_nu");
+    const auto& pp = b.I("prod_ptr");
+    const auto& ps = b.I("prod_species");
+    const auto& pn = b.F("prod_nu");
+    const bool ford = b.f.count("ford_val") != 0;
+    std::vector<char> other(nr, 0);   // extended PLOG and extended fall-off reactions
+    for (const char* k : {"xplog_rxn", "xfo_rxn"})
+      if (b.i.count(k))
+        for (int j : b.I(k)) other.at(j) = 1;
+    dat.assign(4 * (size_t)(nr > 0 ? nr : 1), 0.);
+    pack.assign(4 * (size_t)(nr > 0 ? nr : 1), 0);
+    // one side: its two species, or false when it is not of the packed form
+    auto side = [&](const std::vector<int>& p, const std::vector<int>& sp, const std::vector<double>& v, int j, int* s0,
+                    int* s1, bool* twice) {
+      const int m = p[j + 1] - p[j], q = p[j];
+      *twice = false;
+      *s0 = *s1 = nc;
+      if (m == 1 && (v[q] == 1. || v[q] == 2.)) {
+        *s0 = sp[q];
+        if (v[q] == 2.) { *s1 = sp[q]; *twice = true; }
+        return true;
+      }
+      if (m == 2 && v[q] == 1. && v[q + 1] == 1.) { *s0 = sp[q]; *s1 = sp[q + 1]; return true; }
+      return false;
+    };
+    std::vector<int> rank(nr);
+    for (int j = 0; j < nr; ++j) {
+      int r0, r1, p0, p1;
+      bool rt, pt;
+      bool simple = side(rp, rs, rn, j, &r0, &r1, &rt);
+      simple = side(pp, ps, pn, j, &p0, &p1, &pt) && simple;
+      if (ford) {   // the forward orders are the coefficients
+        const auto& op = b.I("ford_ptr");
+        const int m = rp[j + 1] - rp[j];
+        simple = simple && op[j + 1] - op[j] == m;
+        for (int q = 0; simple && q < m; ++q)
+          simple = b.I("ford_species")[op[j] + q] == rs[rp[j] + q] && b.F("ford_val")[op[j] + q] == rn[rp[j] + q];
+      }
+      simple = simple && rev_kind[j] <= 1 && plog_slot[j] < 0 && cheb_slot[j] < 0 && !other[j];
+      int flags = 0;
+      if (!simple) flags |= kRxSpecial;
+      if (rev_kind[j] == 1) flags |= kRxReversible;
+      if (rt) flags |= kRxTwice;
+      if (b.I("a_sign")[j] < 0) flags |= kRxNegative;
+      dat[4 * j] = b.F("lnA")[j];
+      dat[4 * j + 1] = b.F("beta")[j];
+      dat[4 * j + 2] = b.F("e_over_r")[j];
+      dat[4 * j + 3] = b.F("delta_nu")[j];
+      if (simple) pack[4 * j] = r0 | r1 << 8 | p0 << 16 | p1 << 24;
+      pack[4 * j + 1] = flags;
+      pack[4 * j + 2] = tb_slot[j];
+      pack[4 * j + 3] = fo_slot[j];
+      rank[j] = fo_slot[j] >= 0 ? 0 : !simple ? 1 : tb_slot[j] >= 0 ? 2 : 3;
+    }
+    order.clear();
+    for (int r = 0; r < 4; ++r)
+      for (int j = 0; j < nr; ++j)
+        if (rank[j] == r) order.push_back(j);
+    if (order.empty()) order.push_back(0);
+    ptr.assign(1, 0);
+    ent.clear();
+    for (int i = 0; i < nc; ++i) {
+      for (int j = 0; j < nr; ++j) {
+        auto add = [&](int s, double v, double sign) {
+          if (s != i) return;
+          double word = 0.;   // the reaction in the low half
+          std::memcpy(&word, &j, sizeof(int));
+          ent.push_back(sign * v);
+          ent.push_back(word);
+          if (v != 1. && v != 2.) L.fg_exact = 0;
+        };
+        for (int q = rp[j]; q < rp[j + 1]; ++q) add(rs[q], rn[q], -1.);
+        for (int q = pp[j]; q < pp[j + 1]; ++q) add(ps[q], pn[q], 1.);
+      }
+      ptr.push_back((int)(ent.size() / 2));
+    }
+    if (ent.empty()) ent.assign(2, 0.);
+  }
+  L.rx_dat = B.addd(dat);
+  L.fg_ent = B.addd(ent);
+  L.rx_pack = B.addi(pack);
+  L.rx_order = B.addi(order);
+  L.fg_ptr = B.addi(ptr);
+}
+}  // namespace
+
 bool build_mechanism(const void* blob, size_t nbytes, HostMech& out, std::string& err) {
   Blob b;
   try {
@@ -410,6 +509,7 @@ bool build_mechanism(const void* blob, size_t nbytes, HostMech& out, std::string
       err = "inconsistent array sizes in mechanism blob";
       return false;
     }
+    pack_reactions(b, rev_kind, tb_slot, fo_slot, plog_slot, cheb_slot, B, L);   // the indices have been checked
     while (B.d.size() % 2) B.d.push_back(0.);
     while (B.iv.size() % 4) B.iv.push_back(0);
     L.n_double = (int)B.d.size();
