@@ -76,8 +76,7 @@ struct TransportLayout {
   int eta, lam;               // [nc][4]: ln(eta), ln(lambda) in powers of ln T
   int gam;                    // [n_pair][4]: ln(D_jk P) [m2/s bar] in powers of ln T, pairs j < k row by row
   int teta;                   // [n_teta][nc][4]: theta_ij in powers of T
-  int wilke_phi;              // [nc][nc]: 1 / sqrt(8 (1 + M_k / M_j))
-  int wilke_r14;              // [nc][nc]: (M_j / M_k)^(1/4)
+  int wilke;                  // [nc][nc][2]: sqrt(phi) and sqrt(phi) (M_j / M_k)^(1/4), phi = 1 / sqrt(8 (1 + M_k / M_j))
   // ---- int region
   int iteta;                  // [n_teta] species index of each light species
 };

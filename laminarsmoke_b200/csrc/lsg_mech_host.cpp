@@ -99,11 +99,12 @@ static bool build_transport(const Blob& b, int nc, HostMech& out, std::string& e
   for (int v : it)
     if (v < 0 || v >= nc) { err = "transport species index out of range in mechanism blob"; return false; }
   const std::vector<double>& M = out.mw;
-  std::vector<double> phi((size_t)nc * nc, 0.), r14((size_t)nc * nc, 0.);
+  std::vector<double> wilke((size_t)2 * nc * nc, 0.);
   for (int k = 0; k < nc; ++k)
     for (int j = 0; j < nc; ++j) {
-      phi[(size_t)k * nc + j] = 1. / std::sqrt(8. * (1. + M[k] / M[j]));
-      r14[(size_t)k * nc + j] = std::sqrt(std::sqrt(M[j] / M[k]));
+      const double sphi = std::sqrt(1. / std::sqrt(8. * (1. + M[k] / M[j])));
+      wilke[2 * ((size_t)k * nc + j)] = sphi;
+      wilke[2 * ((size_t)k * nc + j) + 1] = sphi * std::sqrt(std::sqrt(M[j] / M[k]));
     }
   TransportLayout T{};
   T.nc = nc;
@@ -114,8 +115,7 @@ static bool build_transport(const Blob& b, int nc, HostMech& out, std::string& e
   T.lam = B.addd(lam);
   T.gam = B.addd(gam.empty() ? std::vector<double>(2, 0.) : gam);
   T.teta = B.addd(teta.empty() ? std::vector<double>(2, 0.) : teta);
-  T.wilke_phi = B.addd(phi);
-  T.wilke_r14 = B.addd(r14);
+  T.wilke = B.addd(wilke);
   T.iteta = B.addi(it.empty() ? std::vector<int>(1, 0) : it);
   while (B.d.size() % 2) B.d.push_back(0.);
   while (B.iv.size() % 4) B.iv.push_back(0);
@@ -148,6 +148,11 @@ void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::
     const auto& pp = b.I("prod_ptr");
     const auto& ps = b.I("prod_species");
     const auto& pn = b.F("prod_nu");
+    const auto& lnA = b.F("lnA");
+    const auto& beta = b.F("beta");
+    const auto& eor = b.F("e_over_r");
+    const auto& dnu = b.F("delta_nu");
+    const auto& sgn = b.I("a_sign");
     const bool ford = b.f.count("ford_val") != 0;
     std::vector<char> other(nr, 0);   // extended PLOG and extended fall-off reactions
     for (const char* k : {"xplog_rxn", "xfo_rxn"})
@@ -187,11 +192,11 @@ void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::
       if (!simple) flags |= kRxSpecial;
       if (rev_kind[j] == 1) flags |= kRxReversible;
       if (rt) flags |= kRxTwice;
-      if (b.I("a_sign")[j] < 0) flags |= kRxNegative;
-      dat[4 * j] = b.F("lnA")[j];
-      dat[4 * j + 1] = b.F("beta")[j];
-      dat[4 * j + 2] = b.F("e_over_r")[j];
-      dat[4 * j + 3] = b.F("delta_nu")[j];
+      if (sgn[j] < 0) flags |= kRxNegative;
+      dat[4 * j] = lnA[j];
+      dat[4 * j + 1] = beta[j];
+      dat[4 * j + 2] = eor[j];
+      dat[4 * j + 3] = dnu[j];
       if (simple) pack[4 * j] = r0 | r1 << 8 | p0 << 16 | p1 << 24;
       pack[4 * j + 1] = flags;
       pack[4 * j + 2] = tb_slot[j];
@@ -205,19 +210,20 @@ void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::
     if (order.empty()) order.push_back(0);
     ptr.assign(1, 0);
     ent.clear();
+    std::vector<std::vector<double>> rows(nc);   // by species: coefficient, reaction
+    for (int j = 0; j < nr; ++j) {
+      double word = 0.;   // the reaction in the low half
+      std::memcpy(&word, &j, sizeof(int));
+      auto add = [&](int i, double v, double sign) {
+        rows[i].push_back(sign * v);
+        rows[i].push_back(word);
+        if (v != 1. && v != 2.) L.fg_exact = 0;
+      };
+      for (int q = rp[j]; q < rp[j + 1]; ++q) add(rs[q], rn[q], -1.);
+      for (int q = pp[j]; q < pp[j + 1]; ++q) add(ps[q], pn[q], 1.);
+    }
     for (int i = 0; i < nc; ++i) {
-      for (int j = 0; j < nr; ++j) {
-        auto add = [&](int s, double v, double sign) {
-          if (s != i) return;
-          double word = 0.;   // the reaction in the low half
-          std::memcpy(&word, &j, sizeof(int));
-          ent.push_back(sign * v);
-          ent.push_back(word);
-          if (v != 1. && v != 2.) L.fg_exact = 0;
-        };
-        for (int q = rp[j]; q < rp[j + 1]; ++q) add(rs[q], rn[q], -1.);
-        for (int q = pp[j]; q < pp[j + 1]; ++q) add(ps[q], pn[q], 1.);
-      }
+      ent.insert(ent.end(), rows[i].begin(), rows[i].end());
       ptr.push_back((int)(ent.size() / 2));
     }
     if (ent.empty()) ent.assign(2, 0.);

@@ -288,3 +288,36 @@ def test_synthetic_transport_120_species():
     assert rc in (0, -3)                                  # LSG_OK with a GPU, LSG_ERR_CUDA without one
     if rc == 0:
         lsg.lib().lsg_mech_destroy(h)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,n", [("h2co", 1), ("h2co", 129), ("ch4", 31), ("syn120t", 33)])
+def test_gpu_properties_tiles_and_extreme_temperatures(cuda, name, n):
+    """Cells around a block's size, tables in shared memory (h2co, ch4) and read from global memory (syn120t), and a
+    cell whose fits' exponents leave the range of the kernel's polynomial exponential: there the library's takes over,
+    without touching the neighbours.  The sums of these fields have terms of one sign: the fits' exponents (below
+    about 40, three roundings each) bound the error at some 1e-14 relative."""
+    import torch
+    from laminarsmoke_b200 import lsg, mech
+    from oracle.properties import OracleProperties
+    data, species = mech.load(name)
+    Y, T, p = _cells(data, species, n, 29)
+    ctx = lsg.ReactionStep(lsg.Mechanism(data))
+    Yd, pd = torch.tensor(np.ascontiguousarray(Y.T), device=cuda), torch.tensor(p, device=cuda)
+    got = {k: v.cpu().numpy() for k, v in ctx.properties_device(Yd, torch.tensor(T, device=cuda), pd).items()}
+    ref = OracleProperties(data).evaluate(Y, T, p)
+    for f in ("X", "MWmix", "mu", "lambda", "cp", "cp_species", "Dmix"):
+        r = ref[f].T if ref[f].ndim == 2 else ref[f]
+        np.testing.assert_allclose(got[f], r, rtol=1e-12, atol=0., err_msg=f)
+    hot = T.copy()
+    hot[n // 2] = 1e-60
+    far = {k: v.cpu().numpy() for k, v in ctx.properties_device(Yd, torch.tensor(hot, device=cuda), pd).items()}
+    with np.errstate(all="ignore"):
+        ref = OracleProperties(data).evaluate(Y, hot, p)
+    for f in ("X", "Dmix", "mu", "lambda"):
+        r = ref[f].T if ref[f].ndim == 2 else ref[f]
+        keep = np.arange(n) != n // 2
+        np.testing.assert_array_equal(far[f][..., keep], got[f][..., keep])
+    for s in range(len(species)):   # binary fits far outside their range: 0, infinite or NaN as the host's exp
+        d, r = far["Dmix"][s, n // 2], ref["Dmix"][n // 2, s]
+        assert np.isnan(d) == np.isnan(r) and (np.isnan(r) or np.isinf(d) == np.isinf(r))
