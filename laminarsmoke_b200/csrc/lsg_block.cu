@@ -46,21 +46,33 @@ __device__ __forceinline__ double conc_factor_k(double nu, double c1) {
   return pow(c1, nu);
 }
 
-// Block-wide sum; every thread receives the total.  red: BT/32 + 1 doubles.
-template <int BT>
-__device__ __forceinline__ double bsum(double v, double* red) {
+// Block-wide sum; every thread receives the total, added in the order of a tree over the warps' tree sums.  One
+// barrier: the partials go to one half of red (2 BT/32 doubles) in turn, which no thread rewrites before the barrier
+// of the next sum, and every thread adds them itself.  NP: the warps that hold values (the others' are zero).
+template <int BT, int NP = BT / 32>
+__device__ __forceinline__ double bsum(double v, double* red, int& turn) {
+#pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(kFull, v, off);
-  const int w = threadIdx.x >> 5;
+  double* r = red + (turn ? BT / 32 : 0);
+  turn ^= 1;
+  if ((threadIdx.x & 31) == 0) r[threadIdx.x >> 5] = v;
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[w] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    double s = threadIdx.x < BT / 32 ? red[threadIdx.x] : 0.;
-    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(kFull, s, off);
-    if (threadIdx.x == 0) red[BT / 32] = s;
-  }
-  __syncthreads();
-  return red[BT / 32];
+  double s[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) s[i] = r[i];
+#pragma unroll
+  for (int o = NP / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < o; ++i) s[i] += s[i + o];
+  return s[0];
+}
+
+// num / den to the last bit for numerators that are often exactly zero (absent species), without the division's
+// slow path; zero, sign and NaN as the division gives them.
+__device__ __forceinline__ double div0(double num, double den) {
+  const bool z = num == 0.;
+  const double q = (z ? 1. : num) / den;
+  return z ? num * q : q;
 }
 
 // Value of thread src in every thread.
@@ -80,19 +92,19 @@ struct BlockShared {
   double* S;     // [NC] s/R
   double* NET;   // [NR] net rates
   double* X;     // [BT] solve vector
-  double* red;   // [BT/32 + 1]
+  double* red;   // [2 BT/32]: bsum's partials
   double* slot;  // [4]: broadcast, cached T, QR, pivot value
   int* PIV;      // [BT]
   int* ival;     // [BT/32 + 1] pivot search scratch
   int* PERM;     // [BT] the factorisation's row interchanges composed: row i of P b is b[PERM[i]]
   // DRG-reduced step only (drg_block_kernel): the reduced <-> full layout exchange and the dropped reactions
   double* DX;           // [BT]
-  unsigned char* DROP;  // [NR]
+  unsigned char* DROP = nullptr;  // [NR]
 };
 
 template <int BT>
 __host__ __device__ inline size_t block_shared_bytes(const MechLayout& L) {
-  return sizeof(double) * (16 * BT + 3 * (size_t)L.nc + (size_t)L.nr + BT + BT / 32 + 1 + 4) +
+  return sizeof(double) * (16 * BT + 3 * (size_t)L.nc + 2 + (size_t)L.nr + BT + 2 * (BT / 32) + 4) +
          sizeof(int) * (2 * BT + BT / 32 + 1) + 64;
 }
 
@@ -120,11 +132,11 @@ __host__ __device__ inline size_t block_ws_doubles(const MechLayout& L) {
 // (split-TF32 operands) and by the solves (partial sums).
 template <int BT>
 __host__ __device__ inline size_t tcl_head_bytes() {
-  return sizeof(double) * (BT + BT / 32 + 1 + 4) + sizeof(int) * (4 * BT + BT / 32 + 1 + 4) + 16;
+  return sizeof(double) * (BT + 2 * (BT / 32) + 4) + sizeof(int) * (4 * BT + BT / 32 + 1 + 4) + 16;
 }
 template <int BT>
 __host__ __device__ inline size_t tcl_union_bytes(const MechLayout& L) {
-  const size_t rhs = sizeof(double) * (3 * (size_t)L.nc + L.nr);
+  const size_t rhs = sizeof(double) * (3 * (size_t)L.nc + 2 + L.nr);
   const size_t inv = sizeof(float) * ((2 * (BT / 128) + 2) * (size_t)tc::kOperandFloats + 64 + 4 * tc::kPanel);
   const size_t sol = sizeof(double) * 5 * (size_t)BT;
   size_t m = rhs > inv ? rhs : inv;
@@ -138,41 +150,164 @@ __host__ __device__ inline size_t tcl_smem_bytes(const MechLayout& L) {
 // ---------------------------------------------------------------------------
 // RHS, block cooperative (thread i < NC owns species i, thread NC owns T).
 // ---------------------------------------------------------------------------
-template <int BT, bool kDrg = false>
-__device__ __noinline__ double rhs_block(const MechLayout& L, const MechView M, const BlockShared& W,
+// The block's mechanism layout, and the places (in doubles of the dynamic shared memory) of what the out-of-line
+// RHS reads and writes there: through pointers it would address them generically.
+__device__ __forceinline__ MechLayout& blk_layout() {
+  __shared__ MechLayout l;
+  return l;
+}
+extern __shared__ __align__(16) unsigned char bsm[];
+struct RhsPlace {
+  int C, H, S, NET, red, slot, drop;   // drop in bytes (DRG)
+};
+__device__ __forceinline__ RhsPlace rhs_place(const BlockShared& W) {
+  const double* b = (const double*)bsm;
+  return RhsPlace{(int)(W.C - b), (int)(W.H - b), (int)(W.S - b), (int)(W.NET - b), (int)(W.red - b), (int)(W.slot - b),
+                  (int)((const unsigned char*)W.DROP - bsm)};
+}
+
+// Net rate over kMod of a reaction outside the packed form (mech.h bx_pack), and its kMod.
+__device__ __noinline__ double general_rate(const double* __restrict__ Md, const int* __restrict__ Mi, int j, int oC,
+                                            const double* __restrict__ karr, const double* __restrict__ ukeq,
+                                            const double* __restrict__ kinf, const double* __restrict__ logf,
+                                            double cTotSum, double T, double Pk) {
+  const MechLayout& L = blk_layout();
+  const MechView M{Md, Mi};
+  const double* C = (const double*)bsm + oC;
+  const int* tbs = M.I(L.tb_slot);
+  const int* fos = M.I(L.fo_slot);
+  const int* rk = M.I(L.rev_kind);
+  const int* op = M.I(L.ford_ptr);     // forward rate-law orders (FORD, else the coefficients)
+  const int* osp = M.I(L.ford_sp);
+  const double* onu = M.D(L.ford_val);
+  const int* pp = M.I(L.prod_ptr);
+  const int* psp = M.I(L.prod_sp);
+  const double* pnu = M.D(L.prod_nu);
+  double kArr = karr[j];
+  if (L.n_xplog > 0) {   // extended PLOG, every call: k depends on the concentrations (KineticsMap_CHEMKIN.hpp:1662-1670)
+    const int xs = M.I(L.xplog_slot)[j];
+    if (xs >= 0) kArr = xplog_k(M, L, xs, T, log(T), Pk, cTotSum, [&](int k) { return C[k]; });
+  }
+  double kMod = kArr;
+  const int tb = tbs[j];
+  if (tb >= 0) {
+    double Mc = cTotSum;
+    const int* tp = M.I(L.tb_ptr);
+    const int* ts = M.I(L.tb_sp);
+    const double* te = M.D(L.tb_eff);
+    for (int q = tp[tb]; q < tp[tb + 1]; ++q) Mc += C[ts[q]] * te[q];
+    kMod *= Mc;
+  }
+  const int fo = fos[j];
+  if (fo >= 0) {
+    double Mc;
+    const int single = M.I(L.fo_single)[fo];
+    if (single < 0) {
+      Mc = cTotSum;
+      const int* fp = M.I(L.fo_ptr);
+      const int* fs = M.I(L.fo_sp);
+      const double* fe = M.D(L.fo_eff);
+      for (int q = fp[fo]; q < fp[fo + 1]; ++q) Mc += C[fs[q]] * fe[q];
+    } else {
+      Mc = C[single] + 1.e-16;
+    }
+    const double kInf = kinf[fo];
+    const double lF = logf[fo];
+    const double Pr = kArr * Mc / kInf;
+    const bool cabr = M.I(L.fo_cabr)[fo] != 0;
+    double wF = 1.;
+    const int ty = M.I(L.fo_type)[fo];
+    if (ty == 1) {
+      double qq;
+      if (Pr > 1.e-32 || cabr) {
+        const double nTroe = 0.75 - 1.27 * lF;
+        const double cTroe = -0.4 - 0.67 * lF;
+        const double sTroe = log10(Pr) + cTroe;
+        qq = sTroe / (nTroe - 0.14 * sTroe);
+      } else {
+        qq = 1. / 0.14;
+      }
+      wF = pow(10., lF / (1. + qq * qq));
+    } else if (ty == 2) {
+      const double l10 = log10(Pr);
+      const double xSRI = 1. / (1. + l10 * l10);
+      wF = pow(lF, xSRI) * M.D(L.fo_d)[fo];
+      const double e = M.D(L.fo_e)[fo];
+      if (e != 0.) wF *= pow(T, e);
+    }
+    // CABR (KineticsMap_CHEMKIN.hpp:1613-1660): k0 (1 / (1 + Pr)) F; fall-off: k_inf (Pr / (1 + Pr)) F
+    if (cabr) kMod *= (1. / (1. + Pr)) * wF;
+    else kMod *= kInf * (Pr / (1. + Pr)) * wF / kArr;
+  }
+  if (L.n_xfo > 0) {     // extended fall-off (KineticsMap_CHEMKIN.hpp:1672-1681)
+    const int xs = M.I(L.xfo_slot)[j];
+    if (xs >= 0) {
+      kArr = xfo_k(M, L, xs, T, cTotSum, [&](int k) { return C[k]; });
+      kMod = kArr;
+    }
+  }
+  double fwd = 1.;
+  for (int q = op[j]; q < op[j + 1]; ++q) fwd *= conc_factor_k(onu[q], C[osp[q]]);
+  double net = fwd;
+  const int kind = rk[j];
+  if (kind != 0) {
+    double rv = 1.;
+    for (int q = pp[j]; q < pp[j + 1]; ++q) rv *= conc_factor_k(pnu[q], C[psp[q]]);
+    if (kind == 1) rv *= ukeq[j];
+    else rv *= ukeq[j] / kArr;
+    net -= rv;
+  }
+  return net * kMod;
+}
+
+template <int BT, bool kDrg = false, int NP = BT / 32>
+__device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restrict__ Md, const int* __restrict__ Mi,
                                          double* __restrict__ karr, double* __restrict__ ukeq,
-                                         double* __restrict__ kinf, double* __restrict__ logf, double yl, double T,
-                                         double P0, int energy, double rho0) {
+                                         double* __restrict__ kinf, double* __restrict__ logf, double yl, double P0,
+                                         int energy, double rho0, int turn) {
+  const MechLayout& L = blk_layout();
+  const MechView M{Md, Mi};
+  double* const C = (double*)bsm + R.C;
+  double* const H = (double*)bsm + R.H;
+  double* const S = (double*)bsm + R.S;
+  double* const NET = (double*)bsm + R.NET;
+  double* const red = (double*)bsm + R.red;
+  double* const slot = (double*)bsm + R.slot;
   const int tid = threadIdx.x;
   const int NC = L.nc, NR = L.nr;
   const double* MW = M.D(L.mw);
   const double mwl = tid < NC ? MW[tid] : 1.;
-  const double u = bsum<BT>(tid < NC ? yl / mwl : 0., W.red);
+  if (tid == NC) slot[0] = yl;
+  const double u = bsum<BT, NP>(tid < NC ? div0(yl, mwl) : 0., red, turn);
+  const double T = slot[0];
   const double MWmix = 1. / u;
   double xl = 0.;
-  if (tid < NC) { xl = MWmix * yl; xl = xl / mwl; }
+  if (tid < NC) { xl = MWmix * yl; xl = div0(xl, mwl); }
   const bool cv = rho0 > 0.;   // constant volume (BatchReactorHomogeneousConstantVolume.H:148-199)
   const double cTot = cv ? rho0 / MWmix : P0 / kRgas / T;
   const double cl = cTot * xl;
   const double rho = cv ? rho0 : cTot * MWmix;
-  const double* TM = M.D(L.t_mid);
   const double T2 = T * T, T3 = T2 * T, T4 = T3 * T, uT = 1. / T;
+  const bool hi = tid < NC && T > M.D(L.t_mid)[tid];
   double hl = 0.;
   if (tid < NC) {
-    const double* A = T > TM[tid] ? M.D(L.dh_ht) + 6 * tid : M.D(L.dh_lt) + 6 * tid;
+    const double* A = (hi ? M.D(L.dh_ht) : M.D(L.dh_lt)) + 6 * tid;
     hl = A[0] + T * A[1] + T2 * A[2] + T3 * A[3] + T4 * A[4] + uT * A[5];
-    W.C[tid] = cl;
-    W.H[tid] = hl;
+    C[tid] = cl;
+    H[tid] = hl;
+  } else if (tid == NC) {
+    C[NC] = 1.;   // the packed reactions' absent second species
   }
-  const double T_old = W.slot[1];
+  const double T_old = slot[1];
   const bool recalc = fabs(T - T_old) / T > 0.;
   if (recalc && tid < NC) {
     const double logT = log(T);
-    const double* A = T > TM[tid] ? M.D(L.ds_ht) + 6 * tid : M.D(L.ds_lt) + 6 * tid;
-    W.S[tid] = A[0] * logT + T * A[1] + T2 * A[2] + T3 * A[3] + T4 * A[4] + A[5];
+    const double* A = (hi ? M.D(L.ds_ht) : M.D(L.ds_lt)) + 6 * tid;
+    S[tid] = A[0] * logT + T * A[1] + T2 * A[2] + T3 * A[3] + T4 * A[4] + A[5];
   }
   __syncthreads();
-  if (tid == 0) W.slot[1] = T;
+  if (tid == 0) slot[1] = T;
+  const int4* bx = (const int4*)M.I(L.bx_pack);
   if (recalc) {
     const double logT = log(T);
     const double lP = log(101325. / kRgas / T);
@@ -189,13 +324,35 @@ __device__ __noinline__ double rhs_block(const MechLayout& L, const MechView M, 
     const int* pp = M.I(L.prod_ptr);
     const int* psp = M.I(L.prod_sp);
     const double* pnu = M.D(L.prod_nu);
+    const int4* bm = (const int4*)M.I(L.bx_merge);
     for (int j = tid; j < NR; j += BT) {
       double k = exp(lnA[j] + beta[j] * logT - eor[j] * uT);
+      const int flags = L.nc > 31 ? bx[j].z : kRxSpecial;
+      if (!(flags & kRxSpecial)) {
+        if (flags & kRxNegative) k *= -1.;
+        karr[j] = k;
+        if (flags & kRxReversible) {
+          // StoichiometricMap::ReactionEnthalpyAndEntropy: species order, reactant first; the coefficients are +-1
+          // and +-2, so the products are exact
+          const int4 m = bm[j];
+          double dh = 0., ds = 0.;
+          auto add = [&](int e) {
+            const double c = __hiloint2double(e & ~0xffff, 0);
+            dh = __fma_rn(c, H[e & 0xffff], dh);
+            ds = __fma_rn(c, S[e & 0xffff], ds);
+          };
+          add(m.x);
+          add(m.y);
+          add(m.z);
+          add(m.w);
+          ukeq[j] = exp(-ds + dh - lP * dnu[j]);
+        }
+        continue;
+      }
       if (sgn[j] < 0) k *= -1.;
       karr[j] = k;
       const int kind = rk[j];
       if (kind == 1) {
-        // StoichiometricMap::ReactionEnthalpyAndEntropy: species order, reactant first
         double dh = 0., ds = 0.;
         int a = rp[j], b = pp[j];
         const int ae = rp[j + 1], be = pp[j + 1];
@@ -203,12 +360,12 @@ __device__ __noinline__ double rhs_block(const MechLayout& L, const MechView M, 
           const int sa = a < ae ? rsp[a] : (1 << 30);
           const int sb = b < be ? psp[b] : (1 << 30);
           if (sa <= sb) {
-            dh -= contrib_k(rnu[a], W.H[sa]);
-            ds -= contrib_k(rnu[a], W.S[sa]);
+            dh -= contrib_k(rnu[a], H[sa]);
+            ds -= contrib_k(rnu[a], S[sa]);
             ++a;
           } else {
-            dh += contrib_k(pnu[b], W.H[sb]);
-            ds += contrib_k(pnu[b], W.S[sb]);
+            dh += contrib_k(pnu[b], H[sb]);
+            ds += contrib_k(pnu[b], S[sb]);
             ++b;
           }
         }
@@ -219,7 +376,7 @@ __device__ __noinline__ double rhs_block(const MechLayout& L, const MechView M, 
       }
     }
     const int* ft = M.I(L.fo_type);
-    for (int k = tid; k < L.n_fo; k += BT) {
+    for (int k = BT - 1 - tid; k < L.n_fo; k += BT) {   // from the block's end: those threads have one reaction less
       kinf[k] = exp(M.D(L.fo_lnA)[k] + M.D(L.fo_beta)[k] * logT - M.D(L.fo_eor)[k] * uT);
       const double a = M.D(L.fo_a)[k], b = M.D(L.fo_b)[k], c = M.D(L.fo_c)[k], d = M.D(L.fo_d)[k];
       if (ft[k] == 1) {
@@ -233,10 +390,10 @@ __device__ __noinline__ double rhs_block(const MechLayout& L, const MechView M, 
       }
     }
   }
+  const double Pk = cv ? cTot * kRgas * T : P0;
   if (L.n_plog > 0 || L.n_cheb > 0) {
     // pressure-logarithmic and Chebyshev reactions: k depends on P too, so every call
     // (KineticsMap_CHEMKIN.hpp:1332-1348)
-    const double Pk = cv ? cTot * kRgas * T : P0;
     const double logTk = log(T);
     const int* prx = M.I(L.plog_rxn);
     __syncthreads();   // after the Arrhenius values other threads wrote above
@@ -244,127 +401,120 @@ __device__ __noinline__ double rhs_block(const MechLayout& L, const MechView M, 
     const int* crx = M.I(L.cheb_rxn);
     for (int k = tid; k < L.n_cheb; k += BT) karr[crx[k]] = cheb_k(M, L, k, T, Pk);
   }
-  const double cTotSum = bsum<BT>(cl, W.red);   // also orders the cache writes above before their reads
+  const double cTotSum = bsum<BT, NP>(cl, red, turn);   // also orders the cache writes above before their reads
   {
+    // fall-off reactions first, then special forms and third bodies: the lanes of a warp mostly share a path
+    const int* ord = M.I(L.bx_order);
     const int* tbs = M.I(L.tb_slot);
     const int* fos = M.I(L.fo_slot);
-    const int* rk = M.I(L.rev_kind);
-    const int* rp = M.I(L.reac_ptr);
-    const int* rsp = M.I(L.reac_sp);
-    const double* rnu = M.D(L.reac_nu);
-    const int* op = M.I(L.ford_ptr);     // forward rate-law orders (FORD, else the coefficients)
-    const int* osp = M.I(L.ford_sp);
-    const double* onu = M.D(L.ford_val);
-    const int* pp = M.I(L.prod_ptr);
-    const int* psp = M.I(L.prod_sp);
-    const double* pnu = M.D(L.prod_nu);
-    for (int j = tid; j < NR; j += BT) {
-      double kArr = karr[j];
-      if (L.n_xplog > 0) {   // extended PLOG, every call: k depends on the concentrations (KineticsMap_CHEMKIN.hpp:1662-1670)
-        const int xs = M.I(L.xplog_slot)[j];
-        if (xs >= 0) kArr = xplog_k(M, L, xs, T, log(T), cv ? cTot * kRgas * T : P0, cTotSum, [&](int k) { return W.C[k]; });
-      }
-      double kMod = kArr;
-      const int tb = tbs[j];
-      if (tb >= 0) {
-        double Mc = cTotSum;
-        const int* tp = M.I(L.tb_ptr);
-        const int* ts = M.I(L.tb_sp);
-        const double* te = M.D(L.tb_eff);
-        for (int q = tp[tb]; q < tp[tb + 1]; ++q) Mc += W.C[ts[q]] * te[q];
-        kMod *= Mc;
-      }
-      const int fo = fos[j];
-      if (fo >= 0) {
-        double Mc;
-        const int single = M.I(L.fo_single)[fo];
-        if (single < 0) {
-          Mc = cTotSum;
-          const int* fp = M.I(L.fo_ptr);
-          const int* fs = M.I(L.fo_sp);
-          const double* fe = M.D(L.fo_eff);
-          for (int q = fp[fo]; q < fp[fo + 1]; ++q) Mc += W.C[fs[q]] * fe[q];
-        } else {
-          Mc = W.C[single] + 1.e-16;
+    for (int e = tid; e < NR; e += BT) {
+      const int j = L.nc > 31 ? ord[e] : e;
+      const int4 r = L.nc > 31 ? bx[j] : make_int4(0, 0, kRxSpecial, 0);
+      double rate;
+      if (r.z & kRxSpecial) {
+        rate = general_rate(Md, Mi, j, R.C, karr, ukeq, kinf, logf, cTotSum, T, Pk);
+      } else {
+        const double kArr = karr[j];
+        double kMod = kArr;
+        const int tb = tbs[j], fo = fos[j];
+        if (tb >= 0) {
+          double Mc = cTotSum;
+          const int* tp = M.I(L.tb_ptr);
+          const int* ts = M.I(L.tb_sp);
+          const double* te = M.D(L.tb_eff);
+          for (int q = tp[tb]; q < tp[tb + 1]; ++q) Mc += C[ts[q]] * te[q];
+          kMod *= Mc;
         }
-        const double kInf = kinf[fo];
-        const double lF = logf[fo];
-        const double Pr = kArr * Mc / kInf;
-        const bool cabr = M.I(L.fo_cabr)[fo] != 0;
-        double wF = 1.;
-        const int ty = M.I(L.fo_type)[fo];
-        if (ty == 1) {
-          double qq;
-          if (Pr > 1.e-32 || cabr) {
-            const double nTroe = 0.75 - 1.27 * lF;
-            const double cTroe = -0.4 - 0.67 * lF;
-            const double sTroe = log10(Pr) + cTroe;
-            qq = sTroe / (nTroe - 0.14 * sTroe);
+        if (fo >= 0) {
+          double Mc;
+          const int single = M.I(L.fo_single)[fo];
+          if (single < 0) {
+            Mc = cTotSum;
+            const int* fp = M.I(L.fo_ptr);
+            const int* fs = M.I(L.fo_sp);
+            const double* fe = M.D(L.fo_eff);
+            for (int q = fp[fo]; q < fp[fo + 1]; ++q) Mc += C[fs[q]] * fe[q];
           } else {
-            qq = 1. / 0.14;
+            Mc = C[single] + 1.e-16;
           }
-          wF = pow(10., lF / (1. + qq * qq));
-        } else if (ty == 2) {
-          const double l10 = log10(Pr);
-          const double xSRI = 1. / (1. + l10 * l10);
-          wF = pow(lF, xSRI) * M.D(L.fo_d)[fo];
-          const double e = M.D(L.fo_e)[fo];
-          if (e != 0.) wF *= pow(T, e);
+          const double kInf = kinf[fo];
+          const double lF = logf[fo];
+          const double Pr = kArr * Mc / kInf;
+          const bool cabr = M.I(L.fo_cabr)[fo] != 0;
+          double wF = 1.;
+          const int ty = M.I(L.fo_type)[fo];
+          if (ty == 1) {
+            double qq;
+            if (Pr > 1.e-32 || cabr) {
+              const double nTroe = 0.75 - 1.27 * lF;
+              const double cTroe = -0.4 - 0.67 * lF;
+              const double sTroe = log10(Pr) + cTroe;
+              qq = sTroe / (nTroe - 0.14 * sTroe);
+            } else {
+              qq = 1. / 0.14;
+            }
+            wF = pow(10., lF / (1. + qq * qq));
+          } else if (ty == 2) {
+            const double l10 = log10(Pr);
+            const double xSRI = 1. / (1. + l10 * l10);
+            wF = pow(lF, xSRI) * M.D(L.fo_d)[fo];
+            const double e = M.D(L.fo_e)[fo];
+            if (e != 0.) wF *= pow(T, e);
+          }
+          // CABR (KineticsMap_CHEMKIN.hpp:1613-1660): k0 (1 / (1 + Pr)) F; fall-off: k_inf (Pr / (1 + Pr)) F
+          if (cabr) kMod *= (1. / (1. + Pr)) * wF;
+          else kMod *= kInf * (Pr / (1. + Pr)) * wF / kArr;
         }
-        // CABR (KineticsMap_CHEMKIN.hpp:1613-1660): k0 (1 / (1 + Pr)) F; fall-off: k_inf (Pr / (1 + Pr)) F
-        if (cabr) kMod *= (1. / (1. + Pr)) * wF;
-        else kMod *= kInf * (Pr / (1. + Pr)) * wF / kArr;
-      }
-      if (L.n_xfo > 0) {     // extended fall-off (KineticsMap_CHEMKIN.hpp:1672-1681)
-        const int xs = M.I(L.xfo_slot)[j];
-        if (xs >= 0) {
-          kArr = xfo_k(M, L, xs, T, cTotSum, [&](int k) { return W.C[k]; });
-          kMod = kArr;
+        double net = C[r.x & 0xffff] * C[r.x >> 16];
+        if (r.z & kRxReversible) {
+          double rv = C[r.y & 0xffff] * C[r.y >> 16];
+          net = __fma_rn(-rv, ukeq[j], net);
         }
+        rate = net * kMod;
       }
-      double fwd = 1.;
-      for (int q = op[j]; q < op[j + 1]; ++q) fwd *= conc_factor_k(onu[q], W.C[osp[q]]);
-      double net = fwd;
-      const int kind = rk[j];
-      if (kind != 0) {
-        double rv = 1.;
-        for (int q = pp[j]; q < pp[j + 1]; ++q) rv *= conc_factor_k(pnu[q], W.C[psp[q]]);
-        if (kind == 1) rv *= ukeq[j];
-        else rv *= ukeq[j] / kArr;
-        net -= rv;
-      }
-      double r = net * kMod;
       if constexpr (kDrg) {
-        if (W.DROP[j]) r = 0.;   // DRG-reduced system: dropped reactions (chemistry_DRG.H)
+        if (bsm[R.drop + j]) rate = 0.;   // DRG-reduced system: dropped reactions (chemistry_DRG.H)
       }
-      W.NET[j] = r;
+      NET[j] = rate;
     }
   }
   __syncthreads();
   double Rl = 0.;
   if (tid < NC) {
-    const int* fp = M.I(L.fr_ptr);
-    const int* fr = M.I(L.fr_rxn);
-    const double* fc = M.D(L.fr_coef);
-    for (int q = fp[tid]; q < fp[tid + 1]; ++q) {
-      const double c = fc[q];
-      Rl += contrib_k(c < 0. ? -c : c, W.NET[fr[q]]) * (c < 0. ? -1. : 1.);
+    if (L.nc > 31 && L.fe_len > 0) {
+      // the coefficients are +-1 and +-2 (exact products); entries interleaved over the species, so that a warp's
+      // loads are one line each
+      const int2* fe = (const int2*)M.I(L.fe_ent) + tid;
+      const int len = M.I(L.fr_ptr)[tid + 1] - M.I(L.fr_ptr)[tid];
+#pragma unroll 8
+      for (int q = 0; q < len; ++q) {
+        const int2 e = fe[(long)q * NC];
+        Rl = __fma_rn(__hiloint2double(e.y, 0), NET[e.x], Rl);
+      }
+    } else {
+      const int* fp = M.I(L.fr_ptr);
+      const int* fr = M.I(L.fr_rxn);
+      const double* fc = M.D(L.fr_coef);
+      for (int q = fp[tid]; q < fp[tid + 1]; ++q) {
+        const double c = fc[q];
+        Rl += contrib_k(c < 0. ? -c : c, NET[fr[q]]) * (c < 0. ? -1. : 1.);
+      }
     }
   }
-  double dyl = tid < NC ? mwl * Rl / rho : 0.;
-  double QR = W.slot[2];
+  double dyl = tid < NC ? div0(mwl * Rl, rho) : 0.;
+  double QR = energy ? 0. : slot[2];
   if (energy) {
     double cpl = 0.;
     if (tid < NC) {
-      const double* A = T > TM[tid] ? M.D(L.cp_ht) + 5 * tid : M.D(L.cp_lt) + 5 * tid;
+      const double* A = (hi ? M.D(L.cp_ht) : M.D(L.cp_lt)) + 5 * tid;
       cpl = A[0] + T * A[1] + T2 * A[2] + T3 * A[3] + T4 * A[4];
     }
-    const double cpm = bsum<BT>(cpl * xl, W.red) * kRgas;
-    const double d = bsum<BT>(Rl * hl, W.red);
+    const double cpm = bsum<BT, NP>(cpl * xl, red, turn) * kRgas;
+    const double d = bsum<BT, NP>(Rl * hl, red, turn);
     QR = -d * kRgas * T;
     if (cv) {
       const double CvMixMass = (cpm - kRgas) / MWmix;
-      const double sumR = bsum<BT>(Rl, W.red);
+      const double sumR = bsum<BT, NP>(Rl, red, turn);
       if (tid == NC) dyl = (QR + kRgas * T * sumR) / (rho0 * CvMixMass);
     } else {
       const double CpMixMass = cpm / MWmix;
@@ -373,9 +523,7 @@ __device__ __noinline__ double rhs_block(const MechLayout& L, const MechView M, 
   } else if (tid == NC) {
     dyl = 0.;
   }
-  __syncthreads();
-  if (tid == 0) W.slot[2] = QR;
-  __syncthreads();
+  if (tid == 0) slot[2] = QR;   // read by thread 0, or (energy off) unchanged
   return dyl;
 }
 
@@ -437,9 +585,12 @@ struct GearBlock {
   enum { M_TO_FACT, M_FACT };
   enum { CONV_FAIL, CONV_OK };
 
-  const MechLayout* L;
+  // warps that hold components: the others' terms of a sum are zero
+  static constexpr int NP = BT / 32;
   MechView M;
   BlockShared W;
+  RhsPlace place;
+  int turn;
   double* J;      // column-major, leading dimension jld, global
   int jld;
   double* G;      // [n][n] factors, global (FP64 form)
@@ -494,21 +645,23 @@ struct GearBlock {
   // f(y) of the system being integrated: the full reactor, or the DRG-reduced one evaluated through the
   // full layout (kept species fixed, dropped reactions at zero rate) and gathered back
   __device__ double eval(double yl) {
+    double df;
     if constexpr (!DRG) {
-      const double T = bcast(yl, ne - 1, W.slot);
-      return rhs_block<BT>(*L, M, W, karr, ukeq, kinf, logf, yl, T, P0, energy, rho0);
+      df = rhs_block<BT, false, NP>(place, M.d, M.i, karr, ukeq, kinf, logf, yl, P0, energy, rho0, turn);
     } else {
       __syncthreads();
       W.DX[tid] = yl;   // reduced layout
       __syncthreads();
       const double T = W.DX[drg_ni];
       const double yf = tid < drg_nc ? (drg_pos >= 0 ? W.DX[drg_pos] : drg_omega) : T;
-      const double df = rhs_block<BT, true>(*L, M, W, karr, ukeq, kinf, logf, yf, T, P0, energy, rho0);
+      df = rhs_block<BT, true, NP>(place, M.d, M.i, karr, ukeq, kinf, logf, yf, P0, energy, rho0, turn);
       __syncthreads();
       W.DX[tid] = df;   // full layout
       __syncthreads();
-      return W.DX[drg_sp];
+      df = W.DX[drg_sp];
     }
+    if (energy && rho0 > 0.) turn ^= 1;   // its sums: two, four with the energy equation, five at constant volume
+    return df;
   }
 
   __device__ double rhs(double yl) {
@@ -518,7 +671,7 @@ struct GearBlock {
 
   __device__ double error_control(double w) {   // OpenSMOKEUtilities.hpp:689-701
     const double c = active ? w * eps : 0.;
-    return sqrt(bsum<BT>(c * c, W.red) / double(ne));
+    return sqrt(bsum<BT, NP>(c * c, W.red, turn) / double(ne));
   }
 
   __device__ __forceinline__ void check_constraints(double& yl) {
@@ -540,10 +693,8 @@ struct GearBlock {
     double hf = BETA * fabs(h) * error_control(fl) * double(ne);
     if (hf < 1.e-10) hf = 1.;
     const int n = ne;
-    for (int j = 0; j < n; ++j) {
-      const double yh = bcast(yl, j, W.slot);
-      const double ej = bcast(eps, j, W.slot);
-      const double mxj = bcast(maxv, j, W.slot);
+    {   // each thread's increment
+      const double yh = yl, ej = eps, mxj = maxv;
       double hJ;
       if (DRG && unconstrained) {   // KernelDense.hpp:111-193 without maximum constraints
         hJ = ETA2 * fabs(fmax(yh, 1. / ej));
@@ -557,6 +708,11 @@ struct GearBlock {
         hJ = fmax(hJ, ZERO_DER);
         if (yh + hJ > mxj) hJ = -hJ;
       }
+      W.X[tid] = hJ;
+    }
+    __syncthreads();
+    for (int j = 0; j < n; ++j) {
+      const double hJ = W.X[j];
       double yp = yl;
       if (tid == j) yp += hJ;
       const double aux = eval(yp);
@@ -967,8 +1123,8 @@ struct GearBlock {
     va *= h;
     va += active ? Z(1) : 0.;
     va = (active ? V(1) : 0.) - va;
-    const double normd = bsum<BT>(active ? fabs(va) : 0., W.red);
-    const double normf = bsum<BT>(active ? fabs(V(1)) : 0., W.red);
+    const double normd = bsum<BT, NP>(active ? fabs(va) : 0., W.red, turn);
+    const double normf = bsum<BT, NP>(active ? fabs(V(1)) : 0., W.red, turn);
     if (normd > 3. * normf + .1 && iterConvergence > 2) {
       if (numberOfSteps > stepOfLastJacobian + 5u) jacobianStatus = JAC_CHANGE;
       hScale = 0.5; odeHStatus = H_DEC; hNextStep = h * hScale;
@@ -1212,9 +1368,10 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
     block_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepOptions o, StepArgs a,
                  double* __restrict__ ws_all, int* queue, int* err) {
   constexpr bool TCL = TC && BT > 128;
-  extern __shared__ __align__(16) unsigned char bsm[];
   __shared__ int s_cell;
   const int tid = threadIdx.x;
+  if (tid == 0) blk_layout() = L;
+  int turn = 0;
   const int NC = L.nc, ne = NC + 1;
   const size_t wsd = block_ws_doubles(L);
   double* ws = ws_all + (size_t)blockIdx.x * wsd;
@@ -1239,7 +1396,7 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
     karr = zv + 16 * BT;
     double* p = (double*)bsm;
     W.X = p; p += BT;
-    W.red = p; p += BT / 32 + 1;
+    W.red = p; p += 2 * (BT / 32);
     W.slot = p; p += 4;
     int* ip = (int*)p;
     W.PIV = ip; ip += BT;
@@ -1253,7 +1410,7 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
     const uint32_t base = ((s0 + (uint32_t)tcl_head_bytes<BT>() + 1023u) & ~1023u) - s0;
     unsigned char* un = bsm + base;
     double* d = (double*)un;
-    W.C = d; d += NC;
+    W.C = d; d += NC + 2;
     W.H = d; d += NC;
     W.S = d; d += NC;
     W.NET = d;
@@ -1269,12 +1426,12 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
     double* p = (double*)bsm;
     W.Z = p; p += 8 * BT;
     W.V = p; p += 8 * BT;
-    W.C = p; p += NC;
+    W.C = p; p += NC + 2;
     W.H = p; p += NC;
     W.S = p; p += NC;
     W.NET = p; p += L.nr;
     W.X = p; p += BT;
-    W.red = p; p += BT / 32 + 1;
+    W.red = p; p += 2 * (BT / 32);
     W.slot = p; p += 4;
     W.PIV = (int*)p;
     W.ival = W.PIV + BT;
@@ -1329,7 +1486,7 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
     if (Tc > o.tmin_chem) {
       double y0 = yl;
       if (tid < NC && y0 < 0.) y0 = 0.;
-      const double sum = bsum<BT>(tid < NC ? y0 : 0., W.red);
+      const double sum = bsum<BT>(tid < NC ? y0 : 0., W.red, turn);
       if (tid < NC) y0 /= sum;
       if (tid == 0) { W.slot[1] = 0.; W.slot[2] = 0.; }
       __syncthreads();
@@ -1341,9 +1498,10 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
       g.tc_hr0 = 0.;
       g.tc_fp64 = false;
       g.tc_sticky = false;
-      g.L = &L;
       g.M = M;
       g.W = W;
+      g.place = rhs_place(W);
+      g.turn = turn;
       g.J = Jp;
       g.jld = jld;
       g.G = Gp;
@@ -1375,6 +1533,7 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
       const double dtc = a.dt ? a.dt[cell] : a.dt_scalar;
       st = g.solve_to(a.t0 + dtc);
       tc_phase = g.tc_phase;
+      turn = g.turn;
       if (g.tc_failed) {
         tc_failed = true;
         if (tid == 0) atomicOr(err, kErrTensorCoreWait);
@@ -1388,7 +1547,7 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
       for (int k = 0; k < NCNT; ++k) a.counters[(size_t)cell * NCNT + k] = 0;
     }
     // solvers/laminarSMOKE/utilities.H:153-200
-    const double s = bsum<BT>(tid < NC ? yf : 0., W.red);
+    const double s = bsum<BT>(tid < NC ? yf : 0., W.red, turn);
     if (tid < NC) a.Y[(size_t)tid * a.ld + cell] = yf / s;
     if (tid == NC && o.energy) a.T[cell] = yf;
     if (tid == 0) {
@@ -1424,8 +1583,9 @@ template <int BT>
 __global__ void __launch_bounds__(BT, BT == 128 ? 4 : (BT == 256 ? 2 : 1))
     drg_block_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepOptions o, StepArgs a, DrgArgs d,
                      double* __restrict__ ws_all) {
-  extern __shared__ __align__(16) unsigned char bsm[];
   const int tid = threadIdx.x;
+  if (tid == 0) blk_layout() = L;
+  int turn = 0;
   const int lane = tid & 31, warp = tid >> 5;
   const int NC = L.nc, NR = L.nr;
   double* ws = ws_all + (size_t)blockIdx.x * block_ws_doubles(L);
@@ -1437,12 +1597,12 @@ __global__ void __launch_bounds__(BT, BT == 128 ? 4 : (BT == 256 ? 2 : 1))
     double* p = (double*)bsm;
     W.Z = p; p += 8 * BT;
     W.V = p; p += 8 * BT;
-    W.C = p; p += NC;
+    W.C = p; p += NC + 2;
     W.H = p; p += NC;
     W.S = p; p += NC;
     W.NET = p; p += L.nr;
     W.X = p; p += BT;
-    W.red = p; p += BT / 32 + 1;
+    W.red = p; p += 2 * (BT / 32);
     W.slot = p; p += 4;
     W.PIV = (int*)p;
     W.ival = W.PIV + BT;
@@ -1464,8 +1624,8 @@ __global__ void __launch_bounds__(BT, BT == 128 ? 4 : (BT == 256 ? 2 : 1))
       // ---- analysis (DRG.hpp:150-273) ----
       if (tid == 0) { W.slot[1] = 0.; W.slot[2] = 0.; }
       __syncthreads();
-      rhs_block<BT>(L, M, W, karr, karr + L.nr, karr + 2 * L.nr, karr + 2 * L.nr + (L.n_fo > 0 ? L.n_fo : 1),
-                    tid < NC ? om : Tc, Tc, a.p, o.energy, 0.);   // W.NET: net rates of progress
+      rhs_block<BT>(rhs_place(W), M.d, M.i, karr, karr + L.nr, karr + 2 * L.nr,
+                    karr + 2 * L.nr + (L.n_fo > 0 ? L.n_fo : 1), tid < NC ? om : Tc, a.p, o.energy, 0., 0);   // W.NET: net rates of progress
       __syncthreads();
       const double eps = d.eps[cell];
       double den = 0.;
@@ -1531,7 +1691,7 @@ __global__ void __launch_bounds__(BT, BT == 128 ? 4 : (BT == 256 ? 2 : 1))
           nd += keep ? 0 : 1;
         }
       }
-      const double ndrop = bsum<BT>((double)nd, W.red);
+      const double ndrop = bsum<BT>((double)nd, W.red, turn);
       // ---- the reduced system: thread l < ni owns the l-th important species, thread ni owns T ----
       const bool imp = tid < NC && IMPF[tid] != 0;
       const unsigned mi = __ballot_sync(kFull, imp);
@@ -1552,9 +1712,10 @@ __global__ void __launch_bounds__(BT, BT == 128 ? 4 : (BT == 256 ? 2 : 1))
       const double y0 = tid < ni ? W.DX[sp] : (tid == ni ? Tc : 0.);
       __syncthreads();
       GearBlock<BT, false, true> g;
-      g.L = &L;
       g.M = M;
       g.W = W;
+      g.place = rhs_place(W);
+      g.turn = turn;
       g.J = Jp;
       g.jld = NC + 1;
       g.G = Gp;
@@ -1604,7 +1765,7 @@ __global__ void __launch_bounds__(BT, BT == 128 ? 4 : (BT == 256 ? 2 : 1))
       __syncthreads();
       const double Tf = W.DX[ni];
       const double yf = pos >= 0 ? W.DX[pos] : om;
-      const double sum = bsum<BT>(tid < NC ? yf : 0., W.red);
+      const double sum = bsum<BT>(tid < NC ? yf : 0., W.red, turn);
       if (tid < NC) a.Y[(size_t)tid * a.ld + cell] = yf / sum;
       if (tid == 0) {
         if (o.energy) a.T[cell] = Tf;
@@ -1737,8 +1898,8 @@ __global__ void __launch_bounds__(BT) rhs_block_kernel(MechLayout L, const unsig
                                                        long ncells, const double* __restrict__ y,
                                                        double* __restrict__ dy, long ld, double p, int energy,
                                                        double* qr, double* __restrict__ ws_all) {
-  extern __shared__ __align__(16) unsigned char bsm[];
   const int tid = threadIdx.x;
+  if (tid == 0) blk_layout() = L;
   const int NC = L.nc;
   double* ws = ws_all + (size_t)blockIdx.x * block_ws_doubles(L);
   const size_t n = NC + 1;
@@ -1751,12 +1912,12 @@ __global__ void __launch_bounds__(BT) rhs_block_kernel(MechLayout L, const unsig
     double* q = (double*)bsm;
     W.Z = q; q += 8 * BT;
     W.V = q; q += 8 * BT;
-    W.C = q; q += NC;
+    W.C = q; q += NC + 2;
     W.H = q; q += NC;
     W.S = q; q += NC;
     W.NET = q; q += L.nr;
     W.X = q; q += BT;
-    W.red = q; q += BT / 32 + 1;
+    W.red = q; q += 2 * (BT / 32);
     W.slot = q; q += 4;
     W.PIV = (int*)q;
     W.ival = W.PIV + BT;
@@ -1767,8 +1928,7 @@ __global__ void __launch_bounds__(BT) rhs_block_kernel(MechLayout L, const unsig
     __syncthreads();
     if (tid == 0) { W.slot[1] = 0.; W.slot[2] = 0.; }
     const double yl = tid <= NC ? y[(size_t)tid * ld + cell] : 0.;
-    const double T = bcast(yl, NC, W.slot);
-    const double d = rhs_block<BT>(L, M, W, karr, ukeq, kinf, logf, yl, T, p, energy, 0.);
+    const double d = rhs_block<BT>(rhs_place(W), M.d, M.i, karr, ukeq, kinf, logf, yl, p, energy, 0., 0);
     if (tid <= NC) dy[(size_t)tid * ld + cell] = d;
     if (tid == 0 && qr) qr[cell] = W.slot[2];
   }

@@ -57,6 +57,13 @@ struct MechLayout {
   int rx_pack;                                               // int [nr][4]: species bytes, kRx* flags, tb slot, fo slot
   int rx_order;                                              // int [nr]: fall-off first, special forms, the rest
   int fg_ptr;                                                // per species CSR of fg_ent: reaction order, reactants first
+  // ---- and for the block form (more than 31 species)
+  int bx_pack;                                               // int [nr][4]: r0 | r1 << 16, p0 | p1 << 16, kRx* flags, 0
+  int bx_merge;                                              // int [nr][4]: reactants and products in species order, each
+                                                             // species | high half-word of the signed coefficient
+  int bx_order;                                              // int [nr]: fall-off, special forms, third bodies, the rest
+  int fe_ent, fe_len;                                        // int [fe_len][nc][2]: entry q of species i's fr list: reaction,
+                                                             // high word of the coefficient; fe_len 0: not exact products
 };
 
 // Packed reaction (rx_pack): up to two reactants and two products with coefficient one, or one with two (named

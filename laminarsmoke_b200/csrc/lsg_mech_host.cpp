@@ -2,6 +2,7 @@
 #include "lsg_mech_host.h"
 
 #include <cmath>
+#include <algorithm>
 #include <cstring>
 #include <map>
 #include <stdexcept>
@@ -132,12 +133,101 @@ static bool build_transport(const Blob& b, int nc, HostMech& out, std::string& e
 }
 
 namespace {
+// High word of a double.
+int high_word(double v) {
+  long long w;
+  std::memcpy(&w, &v, sizeof(w));
+  return (int)(w >> 32);
+}
+
+// The block form's tables (mech.h bx_*, fe_*), for mechanisms of more than 31 species.
+void pack_block(const Blob& b, const std::vector<int>& rev_kind, const std::vector<int>& tb_slot,
+                const std::vector<int>& fo_slot, const std::vector<int>& plog_slot, const std::vector<int>& cheb_slot,
+                Builder& B, MechLayout& L) {
+  const int nc = L.nc, nr = L.nr;
+  const auto& rp = b.I("reac_ptr");
+  const auto& rs = b.I("reac_species");
+  const auto& rn = b.F("reac_nu");
+  const auto& pp = b.I("prod_ptr");
+  const auto& ps = b.I("prod_species");
+  const auto& pn = b.F("prod_nu");
+  const auto& sgn = b.I("a_sign");
+  const bool ford = b.f.count("ford_val") != 0;
+  std::vector<char> other(nr, 0);   // extended PLOG and extended fall-off reactions
+  for (const char* k : {"xplog_rxn", "xfo_rxn"})
+    if (b.i.count(k))
+      for (int j : b.I(k)) other.at(j) = 1;
+  std::vector<int> pack(4 * (size_t)(nr > 0 ? nr : 1), 0), merge(pack.size(), 0), rank(nr), order;
+  auto side = [&](const std::vector<int>& p, const std::vector<int>& sp, const std::vector<double>& v, int j, int* two) {
+    const int m = p[j + 1] - p[j], q = p[j];
+    two[0] = two[1] = nc;
+    if (m == 1 && (v[q] == 1. || v[q] == 2.)) {
+      two[0] = sp[q];
+      if (v[q] == 2.) two[1] = sp[q];
+      return true;
+    }
+    if (m == 2 && v[q] == 1. && v[q + 1] == 1.) { two[0] = sp[q]; two[1] = sp[q + 1]; return true; }
+    return false;
+  };
+  for (int j = 0; j < nr; ++j) {
+    int r[2], p[2];
+    bool simple = side(rp, rs, rn, j, r);
+    simple = side(pp, ps, pn, j, p) && simple;
+    if (ford) {
+      const auto& op = b.I("ford_ptr");
+      const int m = rp[j + 1] - rp[j];
+      simple = simple && op[j + 1] - op[j] == m;
+      for (int q = 0; simple && q < m; ++q)
+        simple = b.I("ford_species")[op[j] + q] == rs[rp[j] + q] && b.F("ford_val")[op[j] + q] == rn[rp[j] + q];
+    }
+    simple = simple && rev_kind[j] <= 1 && plog_slot[j] < 0 && cheb_slot[j] < 0 && !other[j];
+    pack[4 * j] = simple ? r[0] | r[1] << 16 : 0;
+    pack[4 * j + 1] = simple ? p[0] | p[1] << 16 : 0;
+    pack[4 * j + 2] = (simple ? 0 : kRxSpecial) | (rev_kind[j] == 1 ? kRxReversible : 0) | (sgn[j] < 0 ? kRxNegative : 0);
+    if (simple) {   // species order, the reactant first (StoichiometricMap::ReactionEnthalpyAndEntropy)
+      int a = rp[j], c = pp[j], k = 0;
+      while (a < rp[j + 1] || c < pp[j + 1]) {
+        const int sa = a < rp[j + 1] ? rs[a] : 1 << 30, sc = c < pp[j + 1] ? ps[c] : 1 << 30;
+        const bool reac = sa <= sc;
+        merge[4 * j + k++] = (reac ? sa : sc) | (high_word(reac ? -rn[a] : pn[c]) & ~0xffff);
+        if (reac) ++a;
+        else ++c;
+      }
+    }
+    rank[j] = fo_slot[j] >= 0 ? 0 : !simple ? 1 : tb_slot[j] >= 0 ? 2 : 3;
+  }
+  for (int k = 0; k < 4; ++k)
+    for (int j = 0; j < nr; ++j)
+      if (rank[j] == k) order.push_back(j);
+  if (order.empty()) order.push_back(0);
+  const auto& fp = b.I("fr_ptr");
+  const auto& fr = b.I("fr_rxn");
+  const auto& fc = b.F("fr_coef");
+  int len = 0;
+  for (int i = 0; i < nc; ++i) len = std::max(len, fp[i + 1] - fp[i]);
+  for (double c : fc)   // products with these are exact
+    if (c != 1. && c != -1. && c != 2. && c != -2.) len = 0;
+  std::vector<int> fe(2 * (size_t)(len > 0 ? len * (size_t)nc : 1), 0);
+  if (len > 0)
+    for (int i = 0; i < nc; ++i)
+      for (int q = fp[i]; q < fp[i + 1]; ++q) {
+        fe[2 * ((size_t)(q - fp[i]) * nc + i)] = fr[q];
+        fe[2 * ((size_t)(q - fp[i]) * nc + i) + 1] = high_word(fc[q]);
+      }
+  L.bx_pack = B.addi(pack);
+  L.bx_merge = B.addi(merge);
+  L.bx_order = B.addi(order);
+  L.fe_ent = B.addi(fe);
+  L.fe_len = len;
+}
+
 // The packed reaction table and the reaction-ordered formation-rate lists (mech.h rx_*, fg_*), for mechanisms
 // of up to 31 species; larger ones get empty tables.
 void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::vector<int>& tb_slot,
                     const std::vector<int>& fo_slot, const std::vector<int>& plog_slot,
                     const std::vector<int>& cheb_slot, Builder& B, MechLayout& L) {
   const int nc = L.nc, nr = L.nr;
+  if (L.nc > 31) pack_block(b, rev_kind, tb_slot, fo_slot, plog_slot, cheb_slot, B, L);
   std::vector<double> dat(4, 0.), ent(2, 0.);
   std::vector<int> pack(4, 0), order(1, 0), ptr(1, 0);
   L.fg_exact = 1;
