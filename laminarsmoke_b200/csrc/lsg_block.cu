@@ -11,8 +11,10 @@
 //
 // Per-block work space in HBM: Jacobian J and factors G, both n x n stored by
 // columns (element (i, j) at [j * n + i], so that the threads of a block, one
-// per row, read a column in one coalesced sweep), cached kinetic constants; in shared memory: the Nordsieck arrays, concentrations,
-// enthalpies, entropies, net rates and the pivots.
+// per row, read a column in one coalesced sweep), cached kinetic constants; in
+// shared memory: the Nordsieck arrays, concentrations, enthalpies, entropies,
+// net rates, the pivots, and the factors too where FP64 ones fit (up to 128
+// components).
 #include "lsg_common.cuh"
 #include "lsg_kernels.h"
 #include "lsg_tc.cuh"
@@ -106,6 +108,16 @@ template <int BT>
 __host__ __device__ inline size_t block_shared_bytes(const MechLayout& L) {
   return sizeof(double) * (16 * BT + 3 * (size_t)L.nc + 2 + (size_t)L.nr + BT + 2 * (BT / 32) + 4) +
          sizeof(int) * (2 * BT + BT / 32 + 1) + 64;
+}
+
+// The factors of SG and their work arrays (GearBlock::lu_*), in doubles: G, U, P, R, candidates, flags.
+__host__ __device__ inline size_t shared_lu_doubles(int n) {
+  const size_t ld = (size_t)((n + 3) & ~3);
+  return ld * ld + 8 * ld + 64 + 256 + 16 + 64;
+}
+template <int BT>
+__host__ __device__ inline size_t block_sg_bytes(const MechLayout& L) {
+  return sizeof(double) * shared_lu_doubles(L.nc + 1) + block_shared_bytes<BT>(L) - sizeof(double) * 16 * (BT - 128);
 }
 
 // Threads of the block form: one per ODE component, in whole warpgroups.
@@ -577,7 +589,8 @@ __device__ __forceinline__ double gemv_block(const T* __restrict__ A, int n, con
 // Gear / multivalue BDF integrator for one block (one cell).
 // ---------------------------------------------------------------------------
 // DRG: the DRG-reduced system (chemistry_DRG.H) instead of the full reactor (FP64 factors only).
-template <int BT, bool TC = false, bool DRG = false>
+// SG: FP64 factors of up to 128 components in shared memory, BT > 128 threads a cell (factorize_shared).
+template <int BT, bool TC = false, bool DRG = false, bool SG = false>
 struct GearBlock {
   enum { H_DEC, H_CONST, H_INC };
   enum { O_DEC, O_CONST, O_INC };
@@ -586,7 +599,8 @@ struct GearBlock {
   enum { CONV_FAIL, CONV_OK };
 
   // warps that hold components: the others' terms of a sum are zero
-  static constexpr int NP = BT / 32;
+  static constexpr int NP = SG ? 4 : BT / 32;
+  static constexpr int ZS = SG ? 128 : BT;   // stride of the Nordsieck rows
   MechView M;
   BlockShared W;
   RhsPlace place;
@@ -639,8 +653,8 @@ struct GearBlock {
   int drg_ni = 0, drg_sp = 0, drg_pos = -1, drg_nc = 0;
   double drg_omega = 0.;
 
-  __device__ __forceinline__ double& Z(int i) { return W.Z[i * BT + tid]; }
-  __device__ __forceinline__ double& V(int i) { return W.V[i * BT + tid]; }
+  __device__ __forceinline__ double& Z(int i) { return W.Z[i * ZS + tid]; }
+  __device__ __forceinline__ double& V(int i) { return W.V[i * ZS + tid]; }
 
   // f(y) of the system being integrated: the full reactor, or the DRG-reduced one evaluated through the
   // full layout (kept species fixed, dropped reactions at zero rate) and gathered back
@@ -747,7 +761,385 @@ struct GearBlock {
     }
   }
 
+  // ---- factors in shared memory (SG) ----
+  // The LU of build_and_factorize_fp64, element by element the same operations in the same order, in panels of 8
+  // columns: the panel's rows in the registers of 128 threads (one row each, one barrier of those a pivot), the
+  // panel's rows of U one column a thread, then the trailing matrix by all threads, eight pivots a pass.  Rows stay
+  // where they are until the end (pos: their place in the pivoted order, which decides ties); the last pass puts
+  // them in pivot order.  What bounds it: the chain of a pivot (search, broadcast, division, update), some 1000
+  // cycles of one warp a scheduler.  121 components: 210 thousand cycles (pivots 121, trailing matrix 45, reading J
+  // 24).
+  // In the dynamic shared memory from its start: G [ld][ld] by columns (rows and columns from n on are those of the
+  // unit matrix), U [ld][8] the panel's rows of U, P [2][4][8] the warps' candidate rows, R [2][128] 1 / pivots and
+  // what they lack of it, cand [2][4] the candidates' magnitude (two words), place and row, done [128] the rows
+  // already pivoted.
+  bool recip;   // every pivot's reciprocal is far from overflow and underflow
+  __device__ __forceinline__ static int lu_ld(int n) { return (n + 3) & ~3; }
+  __device__ __forceinline__ static double* lu_g() { return (double*)bsm; }
+  __device__ __forceinline__ static double* lu_u(int n) { return lu_g() + lu_ld(n) * lu_ld(n); }
+  __device__ __forceinline__ static double* lu_p(int n) { return lu_u(n) + 8 * lu_ld(n); }
+  __device__ __forceinline__ static double* lu_r(int n) { return lu_p(n) + 64; }
+  __device__ __forceinline__ static int4* lu_cand(int n) { return (int4*)(lu_r(n) + 256); }
+  __device__ __forceinline__ static int* lu_done(int n) { return (int*)(lu_r(n) + 256 + 16); }
+
+  __device__ __forceinline__ static void bar128() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+  __device__ __noinline__ static bool factorize_shared(int n, const double* J, int jld, double hr0, int perm_at) {
+    const int tid = threadIdx.x, ld = lu_ld(n), r = tid & 127, grp = tid >> 7;
+    const int lane = tid & 31, warp = tid >> 5;
+    double* const G = lu_g();
+    double* const U = lu_u(n);
+    double* const P = lu_p(n);
+    int4* const cand = lu_cand(n);
+    int* const done_s = lu_done(n);
+    int* const prow = (int*)bsm + perm_at;   // physical row of each pivot
+    const double* const Jr = J + r;
+#pragma unroll 16
+    for (int j = grp; j < ld; j += BT / 128) {
+      if (r < ld) {
+        double g = r == j ? 1. : 0.;
+        if (r < n && j < n) {
+          g = __dmul_rn(Jr[(long)j * jld], -hr0);
+          if (r == j) g = __dadd_rn(g, 1.);
+        }
+        G[j * ld + r] = g;
+      }
+    }
+    __syncthreads();
+    int pos = r, buf = 0;
+    bool done = r >= n;
+    for (int k0 = 0; k0 < n; k0 += 8) {
+      const int nb = n - k0 < 8 ? n - k0 : 8;
+      if (tid < 128) {
+        double p[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) p[c] = (c < nb && r < n) ? G[(k0 + c) * ld + r] : 0.;
+        // the current column is always p[0], so that the loop stays small: each pivot shifts the others down
+#pragma unroll 1
+        for (int k = k0; k < k0 + nb; ++k) {
+          // largest magnitude among the rows not yet pivoted, the first place on ties; each warp publishes its best
+          // row, so that one barrier a pivot is enough
+          const unsigned hi = done ? 0u : ((unsigned)__double2hiint(p[0]) & 0x7fffffffu) + 1u;
+          const unsigned lo = (unsigned)__double2loint(p[0]);
+          const unsigned mh = __reduce_max_sync(kFull, hi);
+          unsigned cd = __ballot_sync(kFull, hi == mh);
+          if (cd & (cd - 1u)) {
+            const unsigned ml = __reduce_max_sync(kFull, hi == mh ? lo : 0u);
+            const bool eq = hi == mh && lo == ml;
+            const int pm = __reduce_min_sync(kFull, eq ? pos : 1 << 20);
+            cd = __ballot_sync(kFull, eq && pos == pm);
+          }
+          if (lane == __ffs(cd) - 1) {
+            cand[4 * buf + warp] = make_int4((int)mh, (int)lo, pos, r);
+            double2* q = (double2*)(P + 8 * (4 * buf + warp));
+#pragma unroll
+            for (int c = 0; c < 8; c += 2) q[c >> 1] = make_double2(p[c], p[c + 1]);
+          }
+          bar128();
+          int4 b = cand[4 * buf];
+          int bw = 0;
+#pragma unroll
+          for (int w = 1; w < 4; ++w) {
+            const int4 c = cand[4 * buf + w];
+            const unsigned ch = (unsigned)c.x, bh = (unsigned)b.x, cl = (unsigned)c.y, bl = (unsigned)b.y;
+            if (ch > bh || (ch == bh && (cl > bl || (cl == bl && c.z < b.z)))) { b = c; bw = w; }
+          }
+          const double2* u = (const double2*)(P + 8 * (4 * buf + bw));
+          buf ^= 1;
+          if (!done && pos == k) pos = b.z;
+          if (r == b.w) {
+            pos = k;
+            done = true;
+            prow[k] = r;
+          }
+          const double2 u0 = u[0];
+          double l = p[0];
+          if (!done && u0.x != 0.) l = div0(l, u0.x);
+          if (r < n) G[k * ld + r] = l;
+          if (done) {
+#pragma unroll
+            for (int c = 1; c < 8; ++c) p[c - 1] = p[c];
+          } else {
+            p[0] = __fma_rn(-l, u0.y, p[1]);
+#pragma unroll
+            for (int c = 2; c < 8; c += 2) {
+              const double2 v = u[c >> 1];
+              p[c - 1] = __fma_rn(-l, v.x, p[c]);
+              p[c] = __fma_rn(-l, v.y, p[c + 1]);
+            }
+          }
+          p[7] = 0.;
+        }
+        done_s[r] = done;
+      }
+      __syncthreads();
+      const int j0 = k0 + 8;
+      if (j0 >= n) break;
+      if (tid < n - j0) {
+        double* Gj = G + (j0 + tid) * ld;
+        double u[8];
+        int pr[8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+          pr[m] = prow[k0 + m];
+          u[m] = Gj[pr[m]];
+        }
+#pragma unroll
+        for (int m = 1; m < 8; ++m)
+#pragma unroll
+          for (int q = 0; q < m; ++q) u[m] = __fma_rn(-G[(k0 + q) * ld + pr[m]], u[q], u[m]);
+        double2* Uj = (double2*)(U + 8 * (j0 + tid));
+#pragma unroll
+        for (int m = 0; m < 8; m += 2) Uj[m >> 1] = make_double2(u[m], u[m + 1]);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) Gj[pr[m]] = u[m];
+      }
+      __syncthreads();
+      if (r < n && !done_s[r]) {
+        double l[8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) l[m] = -G[(k0 + m) * ld + r];
+        double* Gr = G + r;
+        int j = j0 + grp;
+        constexpr int kC = 4;   // columns in flight
+        for (; j + (kC - 1) * (BT / 128) < n; j += kC * (BT / 128)) {
+          double g[kC];
+#pragma unroll
+          for (int q = 0; q < kC; ++q) g[q] = Gr[(j + q * (BT / 128)) * ld];
+#pragma unroll
+          for (int m = 0; m < 8; m += 2)
+#pragma unroll
+            for (int q = 0; q < kC; ++q) {
+              const double2 u = *(const double2*)(U + 8 * (j + q * (BT / 128)) + m);
+              g[q] = __fma_rn(l[m], u.x, g[q]);
+              g[q] = __fma_rn(l[m + 1], u.y, g[q]);
+            }
+#pragma unroll
+          for (int q = 0; q < kC; ++q) Gr[(j + q * (BT / 128)) * ld] = g[q];
+        }
+        for (; j < n; j += BT / 128) {
+          double g = Gr[j * ld];
+#pragma unroll
+          for (int m = 0; m < 8; ++m) g = __fma_rn(l[m], U[8 * j + m], g);
+          Gr[j * ld] = g;
+        }
+      }
+      __syncthreads();
+    }
+    // rows into pivot order, a warp a column; then the pivots' reciprocals for the substitution
+    for (int j = warp; j < n; j += BT / 32) {
+      double v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (lane + 32 * q < n) v[q] = G[j * ld + prow[lane + 32 * q]];
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (lane + 32 * q < n) G[j * ld + lane + 32 * q] = v[q];
+      __syncwarp();
+    }
+    __syncthreads();
+    bool far = true;
+    if (tid < 128) {
+      double rd = 1., rl = 0.;
+      if (tid < n) {
+        const double d = G[tid * ld + tid], m = fabs(d);
+        rd = 1. / d;
+        rl = __fma_rn(-d, rd, 1.) * rd;
+        far = m > 1.e-100 && m < 1.e100;
+      }
+      lu_r(n)[tid] = rd;
+      lu_r(n)[128 + tid] = rl;
+    }
+    return __syncthreads_and(far) != 0;
+  }
+
+  // The substitutions of solve_fp64 on the factors in shared memory, by warp 0 alone: lane l holds rows l + 32 q.  Four
+  // columns at a time: their rows' values are broadcast, every lane solves the 4 x 4 triangle for itself (no lane waits
+  // for another one's branch) and applies the four columns, one after the other, to the rows below (above) in its
+  // registers; so every row applies its updates in solve_fp64's order.  Rows whose unknown is out already go on being
+  // updated, which is harmless: the unknowns are kept in X.
+  struct Tri {   // the next four columns: their triangle and, for Q rows of the lane, their entries
+    double2 t[6], r[2], rl[2];
+    double a[4][4];
+  };
+  // Quotient by 1 / d = r + rl (r rounded to nearest, rl the rest): the first estimate is within one unit in the last
+  // place, so the correction by the exact remainder gives the division's own value (Markstein, IBM J. Res. Dev. 34,
+  // 1990) as long as nothing comes near underflow or overflow, which lu_substitute checks afterwards.
+  template <bool kRecip>
+  __device__ __forceinline__ static double quotient(double x, double d, double r, double rl) {
+    if constexpr (!kRecip) return x / d;
+    const double q = __fma_rn(x, r, __dmul_rn(x, rl));
+    return __fma_rn(__fma_rn(-q, d, x), r, q);
+  }
+  template <int Q0, int Q1>
+  __device__ __forceinline__ static void lu_load(Tri& g, const double* G, int ld, int k, int lane) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+#pragma unroll
+      for (int q = Q0; q < Q1; ++q) g.a[c][q] = G[(k + c) * ld + lane + 32 * q];
+    }
+  }
+  __device__ __forceinline__ static void lu_load_lower(Tri& g, const double* G, int ld, int k) {
+    const double* D = G + k * ld + k;
+    g.t[0] = *(const double2*)(D);
+    g.t[1] = *(const double2*)(D + 2);
+    g.t[2] = *(const double2*)(D + ld + 2);
+    g.t[3] = *(const double2*)(D + 2 * ld + 2);
+  }
+  __device__ __forceinline__ static void lu_load_upper(Tri& g, const double* G, const double* R, int ld, int k) {
+    const double* D = G + k * ld + k;
+    g.t[0] = *(const double2*)(D);
+    g.t[1] = *(const double2*)(D + ld);
+    g.t[2] = *(const double2*)(D + 2 * ld);
+    g.t[3] = *(const double2*)(D + 2 * ld + 2);
+    g.t[4] = *(const double2*)(D + 3 * ld);
+    g.t[5] = *(const double2*)(D + 3 * ld + 2);
+    g.r[0] = *(const double2*)(R + k);
+    g.r[1] = *(const double2*)(R + k + 2);
+    g.rl[0] = *(const double2*)(R + 128 + k);
+    g.rl[1] = *(const double2*)(R + 128 + k + 2);
+  }
+  template <int Q0, int Q1>
+  __device__ __forceinline__ static void lu_apply(const Tri& g, const double* v, int c, double* x) {
+#pragma unroll
+    for (int q = Q0; q < Q1; ++q) x[q] = __fma_rn(-g.a[c][q], v[c], x[q]);
+  }
+  // the four columns from k on, in the block of 32 rows Q
+  template <int Q>
+  __device__ __forceinline__ static void lu_forward(const Tri& g, int k, int lane, double* x, double* X) {
+    double v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = __shfl_sync(kFull, x[Q], k + c);
+    v[1] = __fma_rn(-g.t[0].y, v[0], v[1]);
+    v[2] = __fma_rn(-g.t[1].x, v[0], v[2]);
+    v[3] = __fma_rn(-g.t[1].y, v[0], v[3]);
+    lu_apply<Q, 4>(g, v, 0, x);
+    v[2] = __fma_rn(-g.t[2].x, v[1], v[2]);
+    v[3] = __fma_rn(-g.t[2].y, v[1], v[3]);
+    lu_apply<Q, 4>(g, v, 1, x);
+    v[3] = __fma_rn(-g.t[3].y, v[2], v[3]);
+    lu_apply<Q, 4>(g, v, 2, x);
+    lu_apply<Q, 4>(g, v, 3, x);
+    if (lane == 0) {
+      *(double2*)(X + k) = make_double2(v[0], v[1]);
+      *(double2*)(X + k + 2) = make_double2(v[2], v[3]);
+    }
+  }
+  template <int Q, bool kRecip>
+  __device__ __forceinline__ static void lu_back(const Tri& g, int k, int lane, double* x, double* X) {
+    double v[4];
+#pragma unroll
+    for (int c = 3; c >= 0; --c) v[c] = __shfl_sync(kFull, x[Q], k + c);
+    v[3] = quotient<kRecip>(v[3], g.t[5].y, g.r[1].y, g.rl[1].y);
+    v[2] = __fma_rn(-g.t[5].x, v[3], v[2]);
+    v[1] = __fma_rn(-g.t[4].y, v[3], v[1]);
+    v[0] = __fma_rn(-g.t[4].x, v[3], v[0]);
+    lu_apply<0, Q + 1>(g, v, 3, x);
+    v[2] = quotient<kRecip>(v[2], g.t[3].x, g.r[1].x, g.rl[1].x);
+    v[1] = __fma_rn(-g.t[2].y, v[2], v[1]);
+    v[0] = __fma_rn(-g.t[2].x, v[2], v[0]);
+    lu_apply<0, Q + 1>(g, v, 2, x);
+    v[1] = quotient<kRecip>(v[1], g.t[1].y, g.r[0].y, g.rl[0].y);
+    v[0] = __fma_rn(-g.t[1].x, v[1], v[0]);
+    lu_apply<0, Q + 1>(g, v, 1, x);
+    v[0] = quotient<kRecip>(v[0], g.t[0].x, g.r[0].x, g.rl[0].x);
+    lu_apply<0, Q + 1>(g, v, 0, x);
+    if (lane == 0) {
+      *(double2*)(X + k) = make_double2(v[0], v[1]);
+      *(double2*)(X + k + 2) = make_double2(v[2], v[3]);
+    }
+  }
+  template <int Q>
+  __device__ __forceinline__ static void lu_forward_block(const double* G, int ld, int lane, double* x, double* X) {
+    const int end = ld < 32 * Q + 32 ? ld : 32 * Q + 32;
+    if (32 * Q >= end) return;
+    Tri g;
+    lu_load_lower(g, G, ld, 32 * Q);
+    lu_load<Q, 4>(g, G, ld, 32 * Q, lane);
+#pragma unroll 2
+    for (int k = 32 * Q; k < end; k += 4) {
+      const int kn = k + 4 < end ? k + 4 : k;
+      Tri h;
+      lu_load_lower(h, G, ld, kn);
+      lu_load<Q, 4>(h, G, ld, kn, lane);
+      lu_forward<Q>(g, k, lane, x, X);
+      g = h;
+    }
+  }
+  template <int Q, bool kRecip>
+  __device__ __forceinline__ static void lu_back_block(const double* G, const double* R, int ld, int lane, double* x,
+                                                       double* X) {
+    const int end = ld < 32 * Q + 32 ? ld : 32 * Q + 32;
+    if (32 * Q >= end) return;
+    Tri g;
+    lu_load_upper(g, G, R, ld, end - 4);
+    lu_load<0, Q + 1>(g, G, ld, end - 4, lane);
+#pragma unroll 2
+    for (int k = end - 4; k >= 32 * Q; k -= 4) {
+      const int kn = k - 4 >= 32 * Q ? k - 4 : k;
+      Tri h;
+      lu_load_upper(h, G, R, ld, kn);
+      lu_load<0, Q + 1>(h, G, ld, kn, lane);
+      lu_back<Q, kRecip>(g, k, lane, x, X);
+      g = h;
+    }
+  }
+  template <bool kRecip>
+  __device__ __forceinline__ static void lu_substitute(int n, int lane, double* x, double* X) {
+    const int ld = lu_ld(n);
+    const double* const G = lu_g();
+    const double* const R = lu_r(n);
+    lu_forward_block<0>(G, ld, lane, x, X);
+    lu_forward_block<1>(G, ld, lane, x, X);
+    lu_forward_block<2>(G, ld, lane, x, X);
+    lu_forward_block<3>(G, ld, lane, x, X);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = X[lane + 32 * q];
+    __syncwarp();
+    lu_back_block<3, kRecip>(G, R, ld, lane, x, X);
+    lu_back_block<2, kRecip>(G, R, ld, lane, x, X);
+    lu_back_block<1, kRecip>(G, R, ld, lane, x, X);
+    lu_back_block<0, kRecip>(G, R, ld, lane, x, X);
+    __syncwarp();
+  }
+  // X [128] and perm at these offsets (in doubles, in ints) of the dynamic shared memory
+  __device__ __noinline__ static double solve_shared(int n, bool recip, double xl, int x_at, int perm_at) {
+    double* const X = (double*)bsm + x_at;
+    const int* const perm = (const int*)bsm + perm_at;
+    const int tid = threadIdx.x;
+    if (tid < 128) X[tid] = tid < n ? xl : 0.;
+    __syncthreads();
+    if (tid < 32) {
+      double x[4], x0[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = x0[q] = tid + 32 * q < n ? X[perm[tid + 32 * q]] : 0.;
+      __syncwarp();
+      bool again = !recip;
+      if (recip) {
+        lu_substitute<true>(n, tid, x, X);
+        // the quotients are exact if neither they nor the products behind them left the range
+        bool ok = true;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const double m = tid + 32 * q < n ? fabs(X[tid + 32 * q]) : 0.;
+          ok = ok && (m == 0. || (m > 1.e-160 && m < 1.e160));
+        }
+        again = !__all_sync(kFull, ok);
+      }
+      if (again) lu_substitute<false>(n, tid, x0, X);
+    }
+    __syncthreads();
+    return tid < n ? X[tid] : 0.;
+  }
+
   __device__ void build_and_factorize_fp64(double hr0) {
+    if constexpr (SG) {
+      recip = factorize_shared(ne, J, jld, hr0, (int)(W.PERM - (int*)bsm));
+      ++cnt[CNT_FACT];
+      return;
+    }
     const int n = ne;
     for (long e = tid; e < (long)n * n; e += BT) {
       const int j = (int)(e / n), i = (int)(e % n);
@@ -924,6 +1316,10 @@ struct GearBlock {
   }
 
   __device__ double solve_fp64(double xl) {
+    if constexpr (SG) {
+      ++cnt[CNT_SOLVE];
+      return solve_shared(ne, recip, xl, (int)(W.X - (double*)bsm), (int)(W.PERM - (int*)bsm));
+    }
     const int n = ne;
     W.X[tid] = tid < n ? xl : 0.;
     __syncthreads();
@@ -1363,8 +1759,8 @@ struct GearBlock {
 // Persistent block-per-cell kernel: blocks take cells from the queue.
 // chemistry_DI.H:92-235: gather, clip and renormalise, integrate, renormalise, scatter.
 // ---------------------------------------------------------------------------
-template <int BT, bool TC>
-__global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 : (BT == 256 ? 2 : 1)))
+template <int BT, bool TC, bool SG = false>
+__global__ void __launch_bounds__(BT, SG ? 1 : TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 : (BT == 256 ? 2 : 1)))
     block_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepOptions o, StepArgs a,
                  double* __restrict__ ws_all, int* queue, int* err) {
   constexpr bool TCL = TC && BT > 128;
@@ -1424,13 +1820,14 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
     ysm = part + 4 * BT;
   } else {
     double* p = (double*)bsm;
-    W.Z = p; p += 8 * BT;
-    W.V = p; p += 8 * BT;
+    if constexpr (SG) p += shared_lu_doubles(ne);   // the factors come first, then X: 16-byte aligned
+    W.X = p; p += BT;
+    W.Z = p; p += 8 * (SG ? 128 : BT);
+    W.V = p; p += 8 * (SG ? 128 : BT);
     W.C = p; p += NC + 2;
     W.H = p; p += NC;
     W.S = p; p += NC;
     W.NET = p; p += L.nr;
-    W.X = p; p += BT;
     W.red = p; p += 2 * (BT / 32);
     W.slot = p; p += 4;
     W.PIV = (int*)p;
@@ -1490,7 +1887,8 @@ __global__ void __launch_bounds__(BT, TC ? (BT == 128 ? 2 : 1) : (BT == 128 ? 4 
       if (tid < NC) y0 /= sum;
       if (tid == 0) { W.slot[1] = 0.; W.slot[2] = 0.; }
       __syncthreads();
-      GearBlock<BT, TC> g;
+      GearBlock<BT, TC, false, SG> g;
+      g.recip = false;
       g.TS = TS;
       g.tmem = tmem;
       g.tc_phase = tc_phase;
@@ -2002,6 +2400,18 @@ cudaError_t block_plan(const MechLayout& L, int sm_count, bool tc, long* nblocks
   return cudaSuccess;
 }
 
+namespace {
+// Whether the FP64 form keeps a cell's factors in shared memory, one block of 256 threads an SM (more threads spill
+// their registers), instead of four blocks of 128 threads with the factors in the L2: whenever they fit, which leaves
+// the other form to more than some 7000 reactions.  Faster at every size and count measured (ms, before and after):
+// 45 components 22.0 and 11.4 at 96 cells, 42.5 and 35.4 at 592, 1986 and 1469 at 30 000; 121 components 18.3 and 6.2
+// at one cell, 88.9 and 60.9 at 592, 694 and 485 at 6000; 800 reactions and 121 components 811 and 357 at 96 cells,
+// 1798 and 1377 at 1200.
+bool shared_factors(const MechLayout& L) {
+  return block_sg_bytes<256>(L) + 2048 <= 227 * 1024;   // 2048: static shared memory and the block's reserve
+}
+}  // namespace
+
 cudaError_t launch_block(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o,
                          const StepArgs& a, double* ws, long nblocks, int* queue, bool tc, int* err,
                          cudaStream_t stream) {
@@ -2018,6 +2428,16 @@ cudaError_t launch_block(const MechLayout& L, const unsigned char* mech_gmem, co
       block_kernel<256, true><<<(unsigned)g, 256, block_smem<256, true>(L), stream>>>(L, mech_gmem, o, a, ws, queue, err);
     else
       block_kernel<512, true><<<(unsigned)g, 512, block_smem<512, true>(L), stream>>>(L, mech_gmem, o, a, ws, queue, err);
+  } else if (bt == 128 && shared_factors(L)) {
+    constexpr int kT = 256;
+    const size_t smem = block_sg_bytes<kT>(L);
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(block_kernel<kT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    g = g < sms ? g : sms;   // one block an SM (nblocks, the work spaces, is at least the SM count)
+    block_kernel<kT, false, true><<<(unsigned)g, kT, smem, stream>>>(L, mech_gmem, o, a, ws, queue, err);
   } else if (bt == 128) {
     block_kernel<128, false><<<(unsigned)g, 128, block_shared_bytes<128>(L), stream>>>(L, mech_gmem, o, a, ws, queue, err);
   } else if (bt == 256) {

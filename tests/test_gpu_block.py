@@ -77,6 +77,18 @@ def test_block_padded_tight(cuda):
     assert np.abs(Yg - Yo).max() <= ATOL_Y
 
 
+@pytest.mark.parametrize("k,ncells", [(18, 5), (21, 1), (22, 149), (49, 3), (82, 3), (105, 3), (113, 5), (114, 3)],
+                         ids=["n33", "n36", "n37", "n64", "n97", "n120", "n128", "n129"])
+def test_block_shared_factors_sizes(cuda, k, ncells):
+    """FP64 factors in shared memory: component counts around the panels of eight columns, the substitution's four
+    columns and the 32 rows of a lane group, the largest that it takes and the first that it does not."""
+    data, Y, T = _padded_states(k, ncells, seed=13)
+    (Yg, Tg, Qg, stg, nsg), (Yo, To, Qo, sto, cnt) = _run(data, Y, T, 1e-6, rtol=1e-10, atol=1e-16)
+    np.testing.assert_array_equal(stg, sto)
+    assert np.abs(Tg - To).max() / To.min() <= RTOL_T
+    assert np.abs(Yg - Yo).max() <= ATOL_Y
+
+
 @pytest.mark.parametrize("name", ["syn120", "syn500"])
 def test_block_rhs_synthetic(cuda, name):
     """Thermo + rates of the 120- and 500-species synthetic mechanisms (800 / 3000
