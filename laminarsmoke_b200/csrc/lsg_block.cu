@@ -357,6 +357,11 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
           add(m.y);
           add(m.z);
           add(m.w);
+          if (flags & kRxLong) {
+            const int4 o = ((const int4*)M.I(L.bx_more))[j];
+            add(o.x);
+            add(o.y);
+          }
           ukeq[j] = exp(-ds + dh - lP * dnu[j]);
         }
         continue;
@@ -478,8 +483,10 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
           else kMod *= kInf * (Pr / (1. + Pr)) * wF / kArr;
         }
         double net = C[r.x & 0xffff] * C[r.x >> 16];
+        if (r.z & kRxLong) net *= C[r.w & 0xffff];
         if (r.z & kRxReversible) {
           double rv = C[r.y & 0xffff] * C[r.y >> 16];
+          if (r.z & kRxLong) rv *= C[r.w >> 16];
           net = __fma_rn(-rv, ukeq[j], net);
         }
         rate = net * kMod;

@@ -25,8 +25,6 @@ struct GearConsts {
   double Ep[6];
 };
 
-constexpr int kPlainWarpsPerBlock = 4;
-
 // Arguments of one reaction-step launch (device pointers).
 struct StepArgs {
   long ncells;

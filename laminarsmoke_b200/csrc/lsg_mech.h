@@ -57,19 +57,23 @@ struct MechLayout {
   int rx_pack;                                               // int [nr][4]: species bytes, kRx* flags, tb slot, fo slot
   int rx_order;                                              // int [nr]: fall-off first, special forms, the rest
   int fg_ptr;                                                // per species CSR of fg_ent: reaction order, reactants first
-  // ---- and for the block form (more than 31 species)
-  int bx_pack;                                               // int [nr][4]: r0 | r1 << 16, p0 | p1 << 16, kRx* flags, 0
+  // ---- and for the warp and block forms
+  int bx_pack;                                               // int [nr][4]: r0 | r1 << 16, p0 | p1 << 16, kRx* flags,
+                                                             // r2 | p2 << 16 (kRxLong)
   int bx_merge;                                              // int [nr][4]: reactants and products in species order, each
                                                              // species | high half-word of the signed coefficient
+  int bx_more;                                               // int [nr][4]: bx_merge's fifth and sixth entry (kRxLong)
   int bx_order;                                              // int [nr]: fall-off, special forms, third bodies, the rest
   int fe_ent, fe_len;                                        // int [fe_len][nc][2]: entry q of species i's fr list: reaction,
                                                              // high word of the coefficient; fe_len 0: not exact products
+  uint32_t packed_bytes;                                     // of the tables above from rx_dat on
 };
 
 // Packed reaction (rx_pack): up to two reactants and two products with coefficient one, or one with two (named
 // twice), an absent second species named nc (concentration 1, g 0), so that the kernels multiply and add without
 // loops or branches.  kRxSpecial: none of that holds, the general tables apply.
-enum : int { kRxSpecial = 1, kRxReversible = 2, kRxTwice = 4, kRxNegative = 8 };
+// bx_pack takes a third species a side (kRxLong), the factors in the order of the product over the species.
+enum : int { kRxSpecial = 1, kRxReversible = 2, kRxTwice = 4, kRxNegative = 8, kRxLong = 16 };
 
 // Fitted transport properties (the packed blob's tr_* arrays), flattened into
 // a table of their own: [double region][int region], offsets in elements.

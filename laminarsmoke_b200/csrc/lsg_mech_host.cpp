@@ -140,7 +140,7 @@ int high_word(double v) {
   return (int)(w >> 32);
 }
 
-// The block form's tables (mech.h bx_*, fe_*), for mechanisms of more than 31 species.
+// The packed reactions of the warp and block forms (mech.h bx_*, fe_*).
 void pack_block(const Blob& b, const std::vector<int>& rev_kind, const std::vector<int>& tb_slot,
                 const std::vector<int>& fo_slot, const std::vector<int>& plog_slot, const std::vector<int>& cheb_slot,
                 Builder& B, MechLayout& L) {
@@ -157,20 +157,25 @@ void pack_block(const Blob& b, const std::vector<int>& rev_kind, const std::vect
   for (const char* k : {"xplog_rxn", "xfo_rxn"})
     if (b.i.count(k))
       for (int j : b.I(k)) other.at(j) = 1;
-  std::vector<int> pack(4 * (size_t)(nr > 0 ? nr : 1), 0), merge(pack.size(), 0), rank(nr), order;
-  auto side = [&](const std::vector<int>& p, const std::vector<int>& sp, const std::vector<double>& v, int j, int* two) {
+  std::vector<int> pack(4 * (size_t)(nr > 0 ? nr : 1), 0), merge(pack.size(), 0), more(pack.size(), 0), rank(nr), order;
+  // one side's factors: a b c of up to three species with coefficient one, a a b and b b a of a squared and a single one
+  // (the square is formed first, as the product over the species does)
+  auto side = [&](const std::vector<int>& p, const std::vector<int>& sp, const std::vector<double>& v, int j, int* f) {
     const int m = p[j + 1] - p[j], q = p[j];
-    two[0] = two[1] = nc;
-    if (m == 1 && (v[q] == 1. || v[q] == 2.)) {
-      two[0] = sp[q];
-      if (v[q] == 2.) two[1] = sp[q];
-      return true;
+    f[0] = f[1] = f[2] = nc;
+    if (m < 1 || m > 3) return false;
+    int k = 0, twice = -1;
+    for (int e = 0; e < m; ++e) {
+      if (v[q + e] == 2. && twice < 0 && m < 3) twice = e;
+      else if (v[q + e] != 1.) return false;
     }
-    if (m == 2 && v[q] == 1. && v[q + 1] == 1.) { two[0] = sp[q]; two[1] = sp[q + 1]; return true; }
-    return false;
+    if (twice >= 0) f[k++] = sp[q + twice], f[k++] = sp[q + twice];
+    for (int e = 0; e < m; ++e)
+      if (e != twice) f[k++] = sp[q + e];
+    return true;
   };
   for (int j = 0; j < nr; ++j) {
-    int r[2], p[2];
+    int r[3], p[3];
     bool simple = side(rp, rs, rn, j, r);
     simple = side(pp, ps, pn, j, p) && simple;
     if (ford) {
@@ -183,13 +188,16 @@ void pack_block(const Blob& b, const std::vector<int>& rev_kind, const std::vect
     simple = simple && rev_kind[j] <= 1 && plog_slot[j] < 0 && cheb_slot[j] < 0 && !other[j];
     pack[4 * j] = simple ? r[0] | r[1] << 16 : 0;
     pack[4 * j + 1] = simple ? p[0] | p[1] << 16 : 0;
-    pack[4 * j + 2] = (simple ? 0 : kRxSpecial) | (rev_kind[j] == 1 ? kRxReversible : 0) | (sgn[j] < 0 ? kRxNegative : 0);
+    pack[4 * j + 3] = simple ? r[2] | p[2] << 16 : 0;
+    pack[4 * j + 2] = (simple ? 0 : kRxSpecial) | (rev_kind[j] == 1 ? kRxReversible : 0) | (sgn[j] < 0 ? kRxNegative : 0) |
+                      (simple && (r[2] != nc || p[2] != nc) ? kRxLong : 0);
     if (simple) {   // species order, the reactant first (StoichiometricMap::ReactionEnthalpyAndEntropy)
       int a = rp[j], c = pp[j], k = 0;
       while (a < rp[j + 1] || c < pp[j + 1]) {
         const int sa = a < rp[j + 1] ? rs[a] : 1 << 30, sc = c < pp[j + 1] ? ps[c] : 1 << 30;
         const bool reac = sa <= sc;
-        merge[4 * j + k++] = (reac ? sa : sc) | (high_word(reac ? -rn[a] : pn[c]) & ~0xffff);
+        (k < 4 ? merge[4 * j + k] : more[4 * j + k - 4]) = (reac ? sa : sc) | (high_word(reac ? -rn[a] : pn[c]) & ~0xffff);
+        ++k;
         if (reac) ++a;
         else ++c;
       }
@@ -216,6 +224,7 @@ void pack_block(const Blob& b, const std::vector<int>& rev_kind, const std::vect
       }
   L.bx_pack = B.addi(pack);
   L.bx_merge = B.addi(merge);
+  L.bx_more = B.addi(more);
   L.bx_order = B.addi(order);
   L.fe_ent = B.addi(fe);
   L.fe_len = len;
@@ -227,7 +236,8 @@ void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::
                     const std::vector<int>& fo_slot, const std::vector<int>& plog_slot,
                     const std::vector<int>& cheb_slot, Builder& B, MechLayout& L) {
   const int nc = L.nc, nr = L.nr;
-  if (L.nc > 31) pack_block(b, rev_kind, tb_slot, fo_slot, plog_slot, cheb_slot, B, L);
+  const size_t before = B.d.size() * sizeof(double) + B.iv.size() * sizeof(int);
+  pack_block(b, rev_kind, tb_slot, fo_slot, plog_slot, cheb_slot, B, L);
   std::vector<double> dat(4, 0.), ent(2, 0.);
   std::vector<int> pack(4, 0), order(1, 0), ptr(1, 0);
   L.fg_exact = 1;
@@ -323,6 +333,7 @@ void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::
   L.rx_pack = B.addi(pack);
   L.rx_order = B.addi(order);
   L.fg_ptr = B.addi(ptr);
+  L.packed_bytes = (uint32_t)(B.d.size() * sizeof(double) + B.iv.size() * sizeof(int) - before);
 }
 }  // namespace
 

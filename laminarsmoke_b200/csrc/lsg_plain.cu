@@ -7,33 +7,61 @@
 #include <math_constants.h>
 
 namespace lsg {
+namespace {
+
+// Up to 16 warps a block, one block an SM: 128 registers a thread without spills, the mechanism once per SM.
+constexpr int kPlainWarps = 16;
+
+// Layout, tables and the block's cell counter; false after a staging time-out.
+__device__ __forceinline__ int& warp_next() {
+  __shared__ int next;
+  return next;
+}
+template <bool kStaged>
+__device__ __forceinline__ bool warp_setup(const MechLayout& L, const unsigned char* mech_gmem, int* err) {
+  __shared__ __align__(8) uint64_t mbar;
+  if (threadIdx.x == 0) {
+    warp_layout() = L;
+    warp_mech().gmem = mech_gmem;
+    warp_next() = 0;
+  }
+  if constexpr (kStaged) return stage_bulk(warp_smem, mech_gmem, L.bytes, &mbar, err);
+  __syncthreads();
+  return true;
+}
+// The warp's work space (in doubles) in the dynamic shared memory
+template <bool kStaged>
+__device__ __forceinline__ int warp_wofs(const MechLayout& L, int ws_doubles) {
+  return (kStaged ? (int)((L.bytes + 15u) / 16u) * 2 : 0) + (int)(threadIdx.x >> 5) * ws_doubles;
+}
+// The warp's next cell: a block owns every gridDim-th cell, its warps take them in turn.
+__device__ __forceinline__ long warp_cell() {
+  int k = 0;
+  if ((threadIdx.x & 31) == 0) k = atomicAdd(&warp_next(), 1);
+  return (long)blockIdx.x + (long)gridDim.x * __shfl_sync(kFull, k, 0);
+}
+}  // namespace
 
 // solvers/laminarSMOKE/unsteady/chemistry_DI.H:92-235: gather, clip and
 // renormalise, integrate, renormalise, scatter; Q is the reactor's QR after
 // the solve (chemistry_DI.H:168).
-__global__ void __launch_bounds__(kPlainWarpsPerBlock * 32, 1)
+template <bool kStaged>
+__global__ void __launch_bounds__(kPlainWarps * 32, 1)
 plain_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepOptions o, StepArgs a,
                   int* err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ MechLayout sL;
-  if (threadIdx.x == 0) sL = L;
-  if (!stage_bulk(smem, mech_gmem, L.bytes, &mbar, err)) return;
-  const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)L.n_double * sizeof(double));
-  const int warp = threadIdx.x >> 5;
+  if (!warp_setup<kStaged>(L, mech_gmem, err)) return;
   const int lane = threadIdx.x & 31;
-  const long cell = (long)blockIdx.x * kPlainWarpsPerBlock + warp;
-  if (cell >= a.ncells) return;
-  double* wsbase = (double*)(smem + ((L.bytes + 15u) & ~15u)) + (size_t)warp * warp_ws_doubles(L);
-  {
-    WarpWS W0 = carve_ws(wsbase, L);
-    if (lane == 0) {
-      W0.SC[0] = 0.; W0.SC[1] = 0.; W0.SC[2] = a.p; W0.SC[3] = o.energy ? 1. : 0.;
-      W0.SC[4] = a.rho ? a.rho[cell] : 0.;
-    }
-    __syncwarp();
+  const int wofs = warp_wofs<kStaged>(L, warp_ws_doubles(L));
+  const WarpWS W = carve_ws((double*)warp_smem + wofs, L);
+#pragma unroll 1
+  for (long cell; (cell = warp_cell()) < a.ncells;) {
+  __syncwarp();
+  if (lane == 0) {
+    W.SC[0] = 0.; W.SC[1] = 0.; W.SC[2] = a.p; W.SC[3] = o.energy ? 1. : 0.;
+    W.SC[4] = a.rho ? a.rho[cell] : 0.;
+    W.SC[5] = div_w(a.p, kRgas);
   }
+  __syncwarp();
 
   const int NC = L.nc;
   const int ne = NC + 1;
@@ -47,14 +75,11 @@ plain_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, Ste
   if (Tc > o.tmin_chem) {
     double y0 = yl;
     if (lane < NC && y0 < 0.) y0 = 0.;
-    const double sum = seq_sum(lane < NC ? y0 : 0., NC);
-    if (lane < NC) y0 /= sum;
-    GearWarp g;
-    g.L = &sL;
-    g.Md = Md;
-    g.Mi = Mi;
-    g.ws = wsbase;
-    g.W = carve_ws(wsbase, L);
+    const double sum = sum_warp((int)(W.X - (double*)warp_smem), lane < NC ? y0 : 0., NC);
+    if (lane < NC) y0 = div_w(y0, sum);
+    GearWarpT<false, kStaged> g;
+    g.W = W;
+    g.wofs = wofs;
     g.lane = lane;
     g.ne = ne;
     g.active = lane < ne;
@@ -82,15 +107,16 @@ plain_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, Ste
     for (int k = 0; k < NCNT; ++k) a.counters[(size_t)cell * NCNT + k] = 0;
   }
   // solvers/laminarSMOKE/utilities.H:153-200
-  const double s = seq_sum(lane < NC ? yf : 0., NC);
+  const double s = sum_warp((int)(W.X - (double*)warp_smem), lane < NC ? yf : 0., NC);
   if (lane < NC) {
-    yf /= s;
+    yf = div_w(yf, s);
     a.Y[(size_t)lane * a.ld + cell] = yf;
   }
   if (lane == NC && o.energy) a.T[cell] = yf;
   if (lane == 0) {
     if (a.status) a.status[cell] = st;
     if (a.nsteps) a.nsteps[cell] = (int)nsteps;
+  }
   }
 }
 
@@ -122,25 +148,21 @@ __global__ void drg_eps_kernel(long ncells, const double* __restrict__ T, DrgArg
   }
 }
 
-__global__ void __launch_bounds__(kPlainWarpsPerBlock * 32, 1)
+template <bool kStaged>
+__global__ void __launch_bounds__(kPlainWarps * 32, 1)
 drg_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepOptions o, StepArgs a, DrgArgs d,
                 int* err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ MechLayout sL;
-  if (threadIdx.x == 0) sL = L;
-  if (!stage_bulk(smem, mech_gmem, L.bytes, &mbar, err)) return;
-  const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)L.n_double * sizeof(double));
-  const MechView M{Md, Mi};
-  const int warp = threadIdx.x >> 5;
+  if (!warp_setup<kStaged>(L, mech_gmem, err)) return;
+  const MechLayout& sL = warp_layout();
+  const MechView M = warp_tables<kStaged>(sL);
   const int lane = threadIdx.x & 31;
-  const long cell = (long)blockIdx.x * kPlainWarpsPerBlock + warp;
-  if (cell >= a.ncells) return;
-  double* wsbase = (double*)(smem + ((L.bytes + 15u) & ~15u)) + (size_t)warp * drg_ws_doubles(L);
-  WarpWS W = carve_ws(wsbase, L);
+  const int wofs = warp_wofs<kStaged>(L, drg_ws_doubles(L));
+  const WarpWS W = carve_ws((double*)warp_smem + wofs, L);
+#pragma unroll 1
+  for (long cell; (cell = warp_cell()) < a.ncells;) {
+  __syncwarp();
   if (lane == 0) {
-    W.SC[0] = 0.; W.SC[1] = 0.; W.SC[2] = a.p; W.SC[3] = o.energy ? 1. : 0.; W.SC[4] = 0.;
+    W.SC[0] = 0.; W.SC[1] = 0.; W.SC[2] = a.p; W.SC[3] = o.energy ? 1. : 0.; W.SC[4] = 0.; W.SC[5] = div_w(a.p, kRgas);
   }
   __syncwarp();
   const int NC = L.nc, NR = L.nr;
@@ -149,7 +171,7 @@ drg_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepO
   int st = 0, nsp = 0, nrx = 0;
   if (Tc > d.min_T) {
     // ---- analysis (DRG.hpp:150-273): rates at the cell's state, then the search from the key species ----
-    rhs_warp<false>(&sL, Md, Mi, wsbase, lane < NC ? om : Tc, Tc);   // W.NET: net rates of progress
+    rhs_warp<false, kStaged>(wofs, lane < NC ? om : Tc, Tc);   // W.NET: net rates of progress
     __syncwarp();
     const double eps = d.eps[cell];
     double den = 0.;   // sum_k |nu_ki r_k|, reactions in ascending order
@@ -215,12 +237,9 @@ drg_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepO
     const int pos = (lane < NC && ((imp >> lane) & 1u)) ? __popc(imp & ((1u << lane) - 1u)) : -1;
     const double ys = __shfl_sync(kFull, om, sp < NC ? sp : 0);
     const double y0 = lane < ni ? ys : (lane == ni ? Tc : 0.);
-    GearWarpT<true> g;
-    g.L = &sL;
-    g.Md = Md;
-    g.Mi = Mi;
-    g.ws = wsbase;
+    GearWarpT<true, kStaged> g;
     g.W = W;
+    g.wofs = wofs;
     g.lane = lane;
     g.ne = ni + 1;
     g.active = lane < ni + 1;
@@ -256,9 +275,9 @@ drg_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepO
     const double yv = __shfl_sync(kFull, g.y, pos >= 0 ? pos : 0);
     const double Tf = __shfl_sync(kFull, g.y, ni);
     double yf = pos >= 0 ? yv : om;
-    const double sum = seq_sum(lane < NC ? yf : 0., NC);
+    const double sum = sum_warp((int)(W.X - (double*)warp_smem), lane < NC ? yf : 0., NC);
     if (lane < NC) {
-      yf /= sum;
+      yf = div_w(yf, sum);
       a.Y[(size_t)lane * a.ld + cell] = yf;
     }
     if (lane == 0) {
@@ -280,48 +299,87 @@ drg_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepO
     if (d.n_species) d.n_species[cell] = nsp;
     if (d.n_reactions) d.n_reactions[cell] = nrx;
   }
+  }
 }
 
 // Standalone right-hand side, one warp per state (same arithmetic as inside the step).
-__global__ void __launch_bounds__(kPlainWarpsPerBlock * 32)
+template <bool kStaged>
+__global__ void __launch_bounds__(kPlainWarps * 32, 1)
 rhs_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, long ncells, const double* __restrict__ y,
                 double* __restrict__ dy, long ld, double p, int energy, double* qr, int* err) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ __align__(8) uint64_t mbar;
-  __shared__ MechLayout sL;
-  if (threadIdx.x == 0) sL = L;
-  if (!stage_bulk(smem, mech_gmem, L.bytes, &mbar, err)) return;
-  const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)L.n_double * sizeof(double));
-  const int warp = threadIdx.x >> 5;
+  if (!warp_setup<kStaged>(L, mech_gmem, err)) return;
   const int lane = threadIdx.x & 31;
-  const long cell = (long)blockIdx.x * kPlainWarpsPerBlock + warp;
-  if (cell >= ncells) return;
-  double* wsbase = (double*)(smem + ((L.bytes + 15u) & ~15u)) + (size_t)warp * warp_ws_doubles(L);
-  WarpWS W = carve_ws(wsbase, L);
-  if (lane == 0) { W.SC[0] = 0.; W.SC[1] = 0.; W.SC[2] = p; W.SC[3] = energy ? 1. : 0.; W.SC[4] = 0.; }
-  __syncwarp();
+  const int wofs = warp_wofs<kStaged>(L, warp_ws_doubles(L));
+  const WarpWS W = carve_ws((double*)warp_smem + wofs, L);
   const int NC = L.nc;
-  const double yl = lane <= NC ? y[(size_t)lane * ld + cell] : 0.;
-  const double T = __shfl_sync(kFull, yl, NC);
-  const double d = rhs_warp<false>(&sL, Md, Mi, wsbase, yl, T);
-  if (lane <= NC) dy[(size_t)lane * ld + cell] = d;
-  if (lane == 0 && qr) qr[cell] = W.SC[1];
+#pragma unroll 1
+  for (long cell; (cell = warp_cell()) < ncells;) {
+    __syncwarp();
+    if (lane == 0) {
+      W.SC[0] = 0.; W.SC[1] = 0.; W.SC[2] = p; W.SC[3] = energy ? 1. : 0.; W.SC[4] = 0.; W.SC[5] = div_w(p, kRgas);
+    }
+    __syncwarp();
+    const double yl = lane <= NC ? y[(size_t)lane * ld + cell] : 0.;
+    const double T = __shfl_sync(kFull, yl, NC);
+    const double d = rhs_warp<false, kStaged>(wofs, yl, T);
+    if (lane <= NC) dy[(size_t)lane * ld + cell] = d;
+    if (lane == 0 && qr) qr[cell] = W.SC[1];
+  }
 }
+
+namespace {
+// Largest dynamic shared memory of the kernels above beside their static one
+constexpr size_t kPlainSmem = 227 * 1024 - 1024;
+
+// The form takes a mechanism when the tables without the packed copies leave room for four work spaces.
+size_t form_bytes(const MechLayout& L, size_t extra) {
+  const int n = L.nc + 1;
+  auto even = [](size_t x) { return (x + 1) & ~(size_t)1; };
+  const size_t ws = 8 * 32 * 2 + even((size_t)n * (n + 1)) * 2 + 32 * 3 + even(L.nr) * 3 +
+                    even(L.n_fo > 0 ? L.n_fo : 1) * 2 + 16 + 6 + extra;
+  return ((L.bytes - L.packed_bytes + 15u) & ~15u) + 4 * ws * sizeof(double);
+}
+
+// Warps a block, and whether the tables are staged beside their work spaces.  They are unless fewer than four warps
+// would be left, as with some 500 reactions: those read them from global memory.
+int plan_warps(const MechLayout& L, int ws_doubles, bool* staged, size_t* smem) {
+  const size_t mech = (L.bytes + 15u) & ~15u, ws = (size_t)ws_doubles * sizeof(double);
+  size_t w = mech < kPlainSmem ? (kPlainSmem - mech) / ws : 0;
+  *staged = w >= 4;
+  if (!*staged) w = kPlainSmem / ws;
+  if (w > (size_t)kPlainWarps) w = kPlainWarps;
+  *smem = (*staged ? mech : 0) + w * ws;
+  return (int)w;
+}
+
+template <typename K, typename... A>
+cudaError_t launch_warps(const MechLayout& L, int ws_doubles, long ncells, K* staged_kernel, K* global_kernel,
+                         cudaStream_t stream, A... args) {
+  bool staged = false;
+  size_t smem = 0;
+  const int warps = plan_warps(L, ws_doubles, &staged, &smem);
+  if (warps < 1) return cudaErrorInvalidValue;
+  K* k = staged ? staged_kernel : global_kernel;
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const long blocks = ncells < sms ? ncells : sms;   // one an SM: a small batch is a cell an SM
+  k<<<(unsigned)blocks, warps * 32, smem, stream>>>(args...);
+  return cudaGetLastError();
+}
+}  // namespace
+
+size_t plain_smem_bytes(const MechLayout& L) { return form_bytes(L, 0); }
+
+size_t drg_smem_bytes(const MechLayout& L) { return form_bytes(L, (size_t)((L.nr + 7) / 8 + 1)); }
 
 cudaError_t launch_rhs_warp(const MechLayout& L, const unsigned char* mech_gmem, long ncells, const double* y,
                             double* dy, long ld, double p, int energy, double* qr, int* err, cudaStream_t stream) {
-  const size_t smem = plain_smem_bytes(L);
-  cudaError_t e = cudaFuncSetAttribute(rhs_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const long blocks = (ncells + kPlainWarpsPerBlock - 1) / kPlainWarpsPerBlock;
-  rhs_warp_kernel<<<(unsigned)blocks, kPlainWarpsPerBlock * 32, smem, stream>>>(L, mech_gmem, ncells, y, dy, ld, p,
-                                                                                 energy, qr, err);
-  return cudaGetLastError();
-}
-
-size_t plain_smem_bytes(const MechLayout& L) {
-  return ((L.bytes + 15u) & ~15u) + (size_t)kPlainWarpsPerBlock * warp_ws_doubles(L) * sizeof(double);
+  if (plain_smem_bytes(L) > 227 * 1024) return cudaErrorInvalidValue;
+  return launch_warps(L, warp_ws_doubles(L), ncells, rhs_warp_kernel<true>, rhs_warp_kernel<false>, stream, L,
+                      mech_gmem, ncells, y, dy, ld, p, energy, qr, err);
 }
 
 cudaError_t upload_gear_plain(const GearConsts& gc) {
@@ -331,12 +389,8 @@ cudaError_t upload_gear_plain(const GearConsts& gc) {
 cudaError_t launch_plain(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o,
                          const StepArgs& a, int* err, cudaStream_t stream) {
   if (a.ncells <= 0) return cudaSuccess;
-  const size_t smem = plain_smem_bytes(L);
-  cudaError_t e = cudaFuncSetAttribute(plain_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  const long blocks = (a.ncells + kPlainWarpsPerBlock - 1) / kPlainWarpsPerBlock;
-  plain_warp_kernel<<<(unsigned)blocks, kPlainWarpsPerBlock * 32, smem, stream>>>(L, mech_gmem, o, a, err);
-  return cudaGetLastError();
+  return launch_warps(L, warp_ws_doubles(L), a.ncells, plain_warp_kernel<true>, plain_warp_kernel<false>, stream, L,
+                      mech_gmem, o, a, err);
 }
 
 cudaError_t launch_drg_eps(long ncells, const double* T, const DrgArgs& d, cudaStream_t stream) {
@@ -345,21 +399,13 @@ cudaError_t launch_drg_eps(long ncells, const double* T, const DrgArgs& d, cudaS
   return cudaGetLastError();
 }
 
-size_t drg_smem_bytes(const MechLayout& L) {
-  return ((L.bytes + 15u) & ~15u) + (size_t)kPlainWarpsPerBlock * drg_ws_doubles(L) * sizeof(double);
-}
-
 cudaError_t launch_drg_plain(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o,
                              const StepArgs& a, const DrgArgs& d, int* err, cudaStream_t stream) {
   if (a.ncells <= 0) return cudaSuccess;
-  const size_t smem = drg_smem_bytes(L);
-  cudaError_t e = cudaFuncSetAttribute(drg_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = launch_drg_eps(a.ncells, a.T, d, stream);
   if (e != cudaSuccess) return e;
-  e = launch_drg_eps(a.ncells, a.T, d, stream);
-  if (e != cudaSuccess) return e;
-  const long blocks = (a.ncells + kPlainWarpsPerBlock - 1) / kPlainWarpsPerBlock;
-  drg_warp_kernel<<<(unsigned)blocks, kPlainWarpsPerBlock * 32, smem, stream>>>(L, mech_gmem, o, a, d, err);
-  return cudaGetLastError();
+  return launch_warps(L, drg_ws_doubles(L), a.ncells, drg_warp_kernel<true>, drg_warp_kernel<false>, stream, L,
+                      mech_gmem, o, a, d, err);
 }
 
 }  // namespace lsg
