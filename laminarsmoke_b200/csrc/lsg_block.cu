@@ -338,15 +338,16 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
     const double* pnu = M.D(L.prod_nu);
     const int4* bm = (const int4*)M.I(L.bx_merge);
     for (int j = tid; j < NR; j += BT) {
-      double k = exp(lnA[j] + beta[j] * logT - eor[j] * uT);
       const int flags = L.nc > 31 ? bx[j].z : kRxSpecial;
+      const int4 m = bm[j];
+      const double nu = dnu[j];
+      double k = exp(lnA[j] + beta[j] * logT - eor[j] * uT);
       if (!(flags & kRxSpecial)) {
         if (flags & kRxNegative) k *= -1.;
         karr[j] = k;
         if (flags & kRxReversible) {
           // StoichiometricMap::ReactionEnthalpyAndEntropy: species order, reactant first; the coefficients are +-1
           // and +-2, so the products are exact
-          const int4 m = bm[j];
           double dh = 0., ds = 0.;
           auto add = [&](int e) {
             const double c = __hiloint2double(e & ~0xffff, 0);
@@ -362,7 +363,7 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
             add(o.x);
             add(o.y);
           }
-          ukeq[j] = exp(-ds + dh - lP * dnu[j]);
+          ukeq[j] = exp(-ds + dh - lP * nu);
         }
         continue;
       }
@@ -427,39 +428,38 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
     for (int e = tid; e < NR; e += BT) {
       const int j = L.nc > 31 ? ord[e] : e;
       const int4 r = L.nc > 31 ? bx[j] : make_int4(0, 0, kRxSpecial, 0);
+      // what the reaction may need, loaded at once: each level of these tables is a wait of its own
+      const double kArr = karr[j], uk = ukeq[j];
+      const int tb = tbs[j], fo = fos[j];
       double rate;
       if (r.z & kRxSpecial) {
         rate = general_rate(Md, Mi, j, R.C, karr, ukeq, kinf, logf, cTotSum, T, Pk);
       } else {
-        const double kArr = karr[j];
         double kMod = kArr;
-        const int tb = tbs[j], fo = fos[j];
-        if (tb >= 0) {
-          double Mc = cTotSum;
-          const int* tp = M.I(L.tb_ptr);
-          const int* ts = M.I(L.tb_sp);
-          const double* te = M.D(L.tb_eff);
-          for (int q = tp[tb]; q < tp[tb + 1]; ++q) Mc += C[ts[q]] * te[q];
-          kMod *= Mc;
-        }
+        const int t0 = tb >= 0 ? M.I(L.tb_ptr)[tb] : 0, t1 = tb >= 0 ? M.I(L.tb_ptr)[tb + 1] : 0;
+        int f0 = 0, f1 = 0, single = -1, ty = 0;
+        double kInf = 1., lF = 0.;
+        bool cabr = false;
         if (fo >= 0) {
-          double Mc;
-          const int single = M.I(L.fo_single)[fo];
-          if (single < 0) {
-            Mc = cTotSum;
-            const int* fp = M.I(L.fo_ptr);
-            const int* fs = M.I(L.fo_sp);
-            const double* fe = M.D(L.fo_eff);
-            for (int q = fp[fo]; q < fp[fo + 1]; ++q) Mc += C[fs[q]] * fe[q];
-          } else {
-            Mc = C[single] + 1.e-16;
-          }
-          const double kInf = kinf[fo];
-          const double lF = logf[fo];
+          single = M.I(L.fo_single)[fo];
+          f0 = M.I(L.fo_ptr)[fo];
+          f1 = M.I(L.fo_ptr)[fo + 1];
+          ty = M.I(L.fo_type)[fo];
+          cabr = M.I(L.fo_cabr)[fo] != 0;
+          kInf = kinf[fo];
+          lF = logf[fo];
+        }
+        auto bath = [&](const int* sp, const double* eff, int q0, int q1) {
+          double Mc = cTotSum;
+#pragma unroll 4
+          for (int q = q0; q < q1; ++q) Mc += C[sp[q]] * eff[q];
+          return Mc;
+        };
+        if (tb >= 0) kMod *= bath(M.I(L.tb_sp), M.D(L.tb_eff), t0, t1);
+        if (fo >= 0) {
+          const double Mc = single < 0 ? bath(M.I(L.fo_sp), M.D(L.fo_eff), f0, f1) : C[single] + 1.e-16;
           const double Pr = kArr * Mc / kInf;
-          const bool cabr = M.I(L.fo_cabr)[fo] != 0;
           double wF = 1.;
-          const int ty = M.I(L.fo_type)[fo];
           if (ty == 1) {
             double qq;
             if (Pr > 1.e-32 || cabr) {
@@ -487,7 +487,7 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
         if (r.z & kRxReversible) {
           double rv = C[r.y & 0xffff] * C[r.y >> 16];
           if (r.z & kRxLong) rv *= C[r.w >> 16];
-          net = __fma_rn(-rv, ukeq[j], net);
+          net = __fma_rn(-rv, uk, net);
         }
         rate = net * kMod;
       }

@@ -182,6 +182,66 @@ __device__ __forceinline__ uint32_t op_offset(int row, int k) {
   return (uint32_t)((row >> 3) * 1024 + (k >> 2) * 128 + (row & 7) * 16 + (k & 3) * 4);
 }
 
+// The elimination of a panel's 32 columns, a row a thread over NW warps (gj_inverse, gj_inverse_large).  a: the row's
+// panel entries; on return its coefficients W of the panel's rank-32 update (the row after the panel minus the row
+// before it, in terms of the pivot rows).  The column being eliminated is always a[0] and the row moves down by one
+// with each pivot, taking in the pivot's coefficient at the end, so that one small loop body serves all pivots: with
+// every pivot unrolled the block spent 6000 cycles on each, most of them waiting for instructions; now 1500 (501
+// components; the whole inverse 5.8 to 2.6 million cycles).
+// red, redi [2][16]: the warps' largest keys and their rows; prow [2][64]: the scaled pivot row.  Returns the panel
+// column that the row became the pivot of, -1: none.
+template <int NW>
+__device__ __forceinline__ int eliminate_panel(float (&a)[kPanel], bool& pivoted, float* red, int* redi, float* prow) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  unsigned* const keys = (unsigned*)red;
+  constexpr int RS = NW <= 4 ? 4 : 16;
+  int mine = -1;
+#pragma unroll 1
+  for (int c = 0; c < kPanel; ++c) {
+    const int buf = c & 1;
+    // pivot: largest magnitude over the rows not yet pivoted, lowest row on ties; a NaN never outranks a number, but
+    // its row stays a candidate
+    const float m = fabsf(a[0]);
+    const unsigned key = pivoted ? 0u : (m != m ? 0u : __float_as_uint(m)) + 1u;
+    const unsigned wm = __reduce_max_sync(0xffffffffu, key);
+    const int first = __ffs(__ballot_sync(0xffffffffu, key == wm)) - 1;
+    if (lane == 0) {
+      keys[buf * RS + warp] = wm;
+      redi[buf * RS + warp] = warp * 32 + first;
+    }
+    __syncthreads();
+    const unsigned k = lane < NW ? keys[buf * RS + lane] : 0u;
+    const unsigned mx = __reduce_max_sync(0xffffffffu, k);
+    const int w = __ffs(__ballot_sync(0xffffffffu, k == mx && lane < NW)) - 1;
+    const int row = redi[buf * RS + w];
+    float4* const pr = (float4*)(prow + buf * 2 * kPanel);
+    if (tid == row) {
+      const float inv = a[0] != 0.f ? 1.f / a[0] : 0.f;
+#pragma unroll
+      for (int j = 0; j + 1 < kPanel; ++j) a[j] = a[j + 1] * inv;
+      a[kPanel - 1] = inv - 1.f;
+#pragma unroll
+      for (int j = 0; j < kPanel; j += 4)
+        pr[j / 4] = make_float4(a[j], a[j + 1], a[j + 2], j + 4 < kPanel ? a[j + 3] : a[j + 3] + 1.f);
+      pivoted = true;
+      mine = c;
+    }
+    __syncthreads();
+    if (tid != row) {
+      const float f = -a[0];
+#pragma unroll
+      for (int j = 0; j < kPanel; j += 4) {
+        const float4 q = pr[j / 4];
+        a[j] = fmaf(f, q.x, a[j + 1]);
+        a[j + 1] = fmaf(f, q.y, a[j + 2]);
+        a[j + 2] = fmaf(f, q.z, a[j + 3]);
+        a[j + 3] = fmaf(f, q.w, j + 4 < kPanel ? a[(j + 4) % kPanel] : 0.f);
+      }
+    }
+  }
+  return mine;
+}
+
 // ---------------------------------------------------------------------------
 // G^-1 for G = I - hr0 J (J: FP64, column-major n x n in global memory,
 // element (i, j) at J[j * n + i]; 32 <= n <= 128).  All 128 threads call it.
@@ -196,25 +256,27 @@ __device__ __noinline__ bool gj_inverse(const double* __restrict__ J, int n, dou
   const int warp = tid >> 5, lane = tid & 31;
   const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
   // ---- [G | I] into TMEM, row tid ----
+  const double* const Jr = J + (tid < n ? tid : 0);
 #pragma unroll 1
   for (int q = 0; q < kCols / 32; ++q) {
     float v[32];
+    if (q < kRows / 32) {
+      double x[32];   // all 32 loads in flight
 #pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      const int col = q * 32 + k;
-      float g;
-      if (col < kRows) {
+      for (int k = 0; k < 32; ++k) x[k] = Jr[(long)(q * 32 + k < n ? q * 32 + k : 0) * n];
+#pragma unroll
+      for (int k = 0; k < 32; ++k) {
+        const int col = q * 32 + k;
+        v[k] = col == tid ? 1.f : 0.f;
         if (tid < n && col < n) {
-          double x = -hr0 * J[(long)col * n + tid];
-          if (col == tid) x += 1.;
-          g = (float)x;
-        } else {
-          g = col == tid ? 1.f : 0.f;
+          double y = -hr0 * x[k];
+          if (col == tid) y += 1.;
+          v[k] = (float)y;
         }
-      } else {
-        g = (col - kRows) == tid ? 1.f : 0.f;
       }
-      v[k] = g;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 32; ++k) v[k] = q * 32 + k - kRows == tid ? 1.f : 0.f;
     }
     tmem_st32(tmem + lane_base + (uint32_t)(q * 32), v);
   }
@@ -233,65 +295,9 @@ __device__ __noinline__ bool gj_inverse(const double* __restrict__ J, int n, dou
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    float v[32], u[32];
-    tmem_ld32(tmem + lane_base + (uint32_t)k0, v);
-#pragma unroll
-    for (int k = 0; k < 32; ++k) u[k] = 0.f;
-    int mine = -1;   // 0..31: this row is the pivot of panel column `mine`
-#pragma unroll
-    for (int c = 0; c < kPanel; ++c) {
-      const int buf = c & 1;
-      // pivot: largest |G(i, k0 + c)| over the rows not yet pivoted, lowest row on ties
-      float best = pivoted ? -1.f : fabsf(v[c]);
-      if (best != best) best = 0.f;   // a NaN never outranks a number, but its row stays a candidate
-      int brow = tid;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-        const int orow = __shfl_xor_sync(0xffffffffu, brow, off);
-        if (ob > best || (ob == best && orow < brow)) { best = ob; brow = orow; }
-      }
-      if (lane == 0) { S.red[buf * 4 + warp] = best; S.redi[buf * 4 + warp] = brow; }
-      __syncthreads();
-      float pb = S.red[buf * 4];
-      int prow_i = S.redi[buf * 4];
-#pragma unroll
-      for (int w = 1; w < 4; ++w) {
-        const float ob = S.red[buf * 4 + w];
-        const int orow = S.redi[buf * 4 + w];
-        if (ob > pb || (ob == pb && orow < prow_i)) { pb = ob; prow_i = orow; }
-      }
-      float* pr = S.prow + buf * 2 * kPanel;
-      if (tid == prow_i) {
-        const float a = v[c];
-        const float inv = a != 0.f ? 1.f / a : 0.f;
-#pragma unroll
-        for (int k = 0; k < 32; ++k)
-          if (k > c) v[k] *= inv;
-#pragma unroll
-        for (int k = 0; k < 32; ++k)
-          if (k < c) u[k] *= inv;
-        u[c] = inv - 1.f;
-        v[c] = 1.f;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          if (k > c) pr[k] = v[k];
-          if (k <= c) pr[kPanel + k] = u[k] + (k == c ? 1.f : 0.f);
-        }
-        pivoted = true;
-        mine = c;
-      }
-      __syncthreads();
-      if (tid != prow_i) {
-        const float m = v[c];
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          if (k > c) v[k] = fmaf(-m, pr[k], v[k]);
-          if (k <= c) u[k] = fmaf(-m, pr[kPanel + k], u[k]);
-        }
-        v[c] = 0.f;
-      }
-    }
+    float u[32];
+    tmem_ld32(tmem + lane_base + (uint32_t)k0, u);
+    const int mine = eliminate_panel<4>(u, pivoted, S.red, S.redi, S.prow);   // this row is the pivot of that column
     if (mine >= 0) {
       my_col = k0 + mine;
       S.pivot_of_row[tid] = my_col;
@@ -431,18 +437,23 @@ __device__ __noinline__ bool gj_inverse_large(const double* __restrict__ J, int 
   const int wg = tid >> 7, r128 = tid & 127;
   const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t col_base = (uint32_t)(wg * 128);
-  // G = I - hr0 J, padded with the identity, row tid of every column
-#pragma unroll 4
-  for (int c = 0; c < NP; ++c) {
-    float g;
-    if (tid < n && c < n) {
-      double x = -hr0 * J[(long)c * jld + tid];
-      if (c == tid) x += 1.;
-      g = (float)x;
-    } else {
-      g = c == tid ? 1.f : 0.f;
+  // G = I - hr0 J, padded with the identity, row tid of every column; 16 columns' loads in flight
+  const double* const Jr = J + (tid < n ? tid : 0);
+#pragma unroll 1
+  for (int c = 0; c < NP; c += 16) {
+    double x[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = Jr[(long)(c + k < n ? c + k : 0) * jld];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      float g = c + k == tid ? 1.f : 0.f;
+      if (tid < n && c + k < n) {
+        double y = -hr0 * x[k];
+        if (c + k == tid) y += 1.;
+        g = (float)y;
+      }
+      R[(long)(c + k) * NP + tid] = g;
     }
-    R[(long)c * NP + tid] = g;
   }
   S.colof[tid] = -1;
   S.piv[tid] = tid;
@@ -454,65 +465,10 @@ __device__ __noinline__ bool gj_inverse_large(const double* __restrict__ J, int 
   for (int pn = 0; pn < npanels; ++pn) {
     const int k0 = pn * kPanel;
     __syncthreads();   // the previous panel's stores of R are visible to the block
-    float v[32], u[32];
+    float u[32];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) v[k] = R[(long)(k0 + k) * NP + tid];
-#pragma unroll
-    for (int k = 0; k < 32; ++k) u[k] = 0.f;
-    int mine = -1;
-#pragma unroll
-    for (int c = 0; c < kPanel; ++c) {
-      const int buf = c & 1;
-      float best = pivoted ? -1.f : fabsf(v[c]);
-      if (best != best) best = 0.f;
-      int brow = tid;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        const float ob = __shfl_xor_sync(0xffffffffu, best, off);
-        const int orow = __shfl_xor_sync(0xffffffffu, brow, off);
-        if (ob > best || (ob == best && orow < brow)) { best = ob; brow = orow; }
-      }
-      if (lane == 0) { S.red[buf * 16 + warp] = best; S.redi[buf * 16 + warp] = brow; }
-      __syncthreads();
-      float pb = S.red[buf * 16];
-      int prow_i = S.redi[buf * 16];
-#pragma unroll
-      for (int w = 1; w < NW; ++w) {
-        const float ob = S.red[buf * 16 + w];
-        const int orow = S.redi[buf * 16 + w];
-        if (ob > pb || (ob == pb && orow < prow_i)) { pb = ob; prow_i = orow; }
-      }
-      float* pr = S.prow + buf * 2 * kPanel;
-      if (tid == prow_i) {
-        const float a = v[c];
-        const float inv = a != 0.f ? 1.f / a : 0.f;
-#pragma unroll
-        for (int k = 0; k < 32; ++k)
-          if (k > c) v[k] *= inv;
-#pragma unroll
-        for (int k = 0; k < 32; ++k)
-          if (k < c) u[k] *= inv;
-        u[c] = inv - 1.f;
-        v[c] = 1.f;
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          if (k > c) pr[k] = v[k];
-          if (k <= c) pr[kPanel + k] = u[k] + (k == c ? 1.f : 0.f);
-        }
-        pivoted = true;
-        mine = c;
-      }
-      __syncthreads();
-      if (tid != prow_i) {
-        const float m = v[c];
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          if (k > c) v[k] = fmaf(-m, pr[k], v[k]);
-          if (k <= c) u[k] = fmaf(-m, pr[kPanel + k], u[k]);
-        }
-        v[c] = 0.f;
-      }
-    }
+    for (int k = 0; k < 32; ++k) u[k] = R[(long)(k0 + k) * NP + tid];
+    const int mine = eliminate_panel<NW>(u, pivoted, S.red, S.redi, S.prow);
     if (mine >= 0) {
       S.colof[tid] = k0 + mine;
       S.piv[k0 + mine] = tid;
@@ -539,26 +495,44 @@ __device__ __noinline__ bool gj_inverse_large(const double* __restrict__ J, int 
     }
     float* const B_hi = S.B;
     float* const B_lo = S.B + kOperandFloats;
+    float* const stage = S.B;        // [32][kStage]: column c of pivot k, before the conversion
+    constexpr int kStage = 136;      // 8 mod 32 banks: a core matrix's 32 words on 32 banks
 #pragma unroll 1
     for (int ch = 0; ch < nchunks; ++ch) {
       const int c0 = ch * 128;
-      // the chunk of this row into TMEM; the pivot rows also write it as the B operand
+      // the chunk of this row into TMEM; the pivot rows also stage it where the B operand goes, to which all threads
+      // then convert it (left to the pivot rows, of which nearly every warp has one, the conversion took every warp
+      // through all of it)
 #pragma unroll 1
       for (int q = 0; q < 4; ++q) {
         float r[32];
 #pragma unroll
         for (int k = 0; k < 32; ++k) r[k] = R[(long)(c0 + q * 32 + k) * NP + tid];
         if (mine >= 0) {
+          float4* st = (float4*)(stage + mine * kStage + q * 32);
 #pragma unroll
-          for (int k = 0; k < 32; ++k) {
-            const float x = r[k];
-            const float xh = __uint_as_float(to_tf32(x));
-            const uint32_t off = op_offset(q * 32 + k, mine);
-            *(float*)((char*)B_hi + off) = xh;
-            *(float*)((char*)B_lo + off) = __uint_as_float(to_tf32(x - xh));
-          }
+          for (int k = 0; k < 32; k += 4) st[k / 4] = make_float4(r[k], r[k + 1], r[k + 2], r[k + 3]);
         }
         tmem_st32(tmem + lane_base + col_base + (uint32_t)(q * 32), r);
+      }
+      __syncthreads();
+      {
+        float x[128 * kPanel / BT];
+        const int k = lane & 3, col = lane >> 2;   // a core matrix (8 columns x 4 pivots) a warp and turn
+#pragma unroll
+        for (int e = 0; e < 128 * kPanel / BT; ++e) {
+          const int m = e * NW + warp;
+          x[e] = stage[((m & 7) * 4 + k) * kStage + (m >> 3) * 8 + col];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < 128 * kPanel / BT; ++e) {
+          const int m = e * NW + warp;
+          const uint32_t off = op_offset((m >> 3) * 8 + col, (m & 7) * 4 + k);
+          const float xh = __uint_as_float(to_tf32(x[e]));
+          *(float*)((char*)B_hi + off) = xh;
+          *(float*)((char*)B_lo + off) = __uint_as_float(to_tf32(x[e] - xh));
+        }
       }
       tmem_wait_st();
       fence_async_smem();
