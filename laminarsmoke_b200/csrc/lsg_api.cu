@@ -1267,7 +1267,7 @@ int lsg_steady_sources_sparse_device(lsg_ctx* c, int ncells, int nspecies, const
                                                      S_implicit, S_explicit, lds, c->sm_count, c->d_err, s);
   if (e == cudaErrorInvalidValue) { cudaGetLastError(); return LSG_ERR_UNSUPPORTED; }
   if (e != cudaSuccess) return LSG_ERR_CUDA;
-  ++c->launches;
+  c->launches += 2;
   return LSG_OK;
 }
 

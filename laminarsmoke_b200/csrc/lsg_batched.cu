@@ -407,10 +407,10 @@ batched_kernel(MechLayout Lp, const unsigned char* __restrict__ mech_gmem, StepO
   __shared__ __align__(8) uint64_t mbar;
   __shared__ MechLayout sL;
   if (threadIdx.x == 0) sL = Lp;
-  if (!stage_bulk(smem, mech_gmem, Lp.bytes, &mbar, err)) return;
+  if (!stage_tables(smem, mech_gmem, Lp, Lp.base_int, &mbar, err)) return;
   const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)Lp.n_double * sizeof(double));
-  double* scratch = (double*)(smem + ((Lp.bytes + 15u) & ~15u));
+  const int* Mi = (const int*)(smem + (size_t)Lp.base_double * sizeof(double));
+  double* scratch = (double*)(smem + staged_bytes(Lp, Lp.base_int));
   const int NC = Lp.nc, n = NC + 1;
   // per-lane shared blocks: Newton correction DB[n][kBT], LU[n*n][kLS], pivots[n][kBT]
   double* sDB = scratch + (size_t)4 * NC * kBT;
@@ -1124,7 +1124,7 @@ __host__ size_t batched_slot_doubles(const MechLayout& L, bool lu64) {
 
 size_t batched_smem_bytes(const MechLayout& L, bool lu64) {
   const size_t n = L.nc + 1;
-  return ((L.bytes + 15u) & ~15u) + (size_t)4 * L.nc * kBT * sizeof(double) + n * kBT * sizeof(double) +
+  return staged_bytes(L, L.base_int) + (size_t)4 * L.nc * kBT * sizeof(double) + n * kBT * sizeof(double) +
          ((n * n * kLS * (lu64 ? sizeof(double) : sizeof(float)) + 15) & ~(size_t)15) + n * kBT * sizeof(int) + 16;
 }
 

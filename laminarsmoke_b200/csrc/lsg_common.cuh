@@ -176,12 +176,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// Stage `bytes` (multiple of 16, both addresses 16-byte aligned) from global
-// to shared memory with one-dimensional bulk copies issued by thread 0 and
-// completed on an mbarrier.  Waits are bounded; on timeout the block's
+// Stage a mechanism's tables (staged_bytes: its doubles before the packed
+// tables and its first `ints` ints, one after the other; every part a multiple
+// of 16 bytes at a 16-byte boundary) from global to shared memory with
+// one-dimensional bulk copies issued by thread 0 and completed on an mbarrier.  Waits are bounded; on timeout the block's
 // error flag is raised and false is returned (the caller must then not use
 // the shared copy).  Must be called by all threads of the block.
-__device__ inline bool stage_bulk(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* mbar, int* err) {
+__device__ inline bool stage_tables(void* smem_dst, const unsigned char* mech, const MechLayout& L, int ints,
+                                    uint64_t* mbar, int* err) {
   const uint32_t bar = smem_u32(mbar);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
@@ -189,15 +191,19 @@ __device__ inline bool stage_bulk(void* smem_dst, const void* gsrc, uint32_t byt
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    const uint32_t split = (uint32_t)L.base_double * 8u, bytes = staged_bytes(L, ints);
+    const uint32_t gap = (uint32_t)(L.n_double - L.base_double) * 8u;   // the packed tables' doubles are left out
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     const uint32_t dst = smem_u32(smem_dst);
     const uint32_t chunk = 32768;   // several copies, each a multiple of 16 bytes
-    for (uint32_t off = 0; off < bytes; off += chunk) {
-      const uint32_t n = (bytes - off) < chunk ? (bytes - off) : chunk;
+    for (uint32_t off = 0; off < bytes;) {
+      const uint32_t end = off < split ? split : bytes;
+      const uint32_t n = (end - off) < chunk ? (end - off) : chunk;
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + off),
-          "l"((const char*)gsrc + off), "r"(n), "r"(bar)
+          "l"((const char*)mech + off + (off < split ? 0u : gap)), "r"(n), "r"(bar)
           : "memory");
+      off += n;
     }
   }
   uint32_t done = 0;

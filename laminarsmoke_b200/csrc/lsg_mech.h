@@ -50,6 +50,9 @@ struct MechLayout {
   int tb_ptr, tb_sp;                                         // third body CSR (by slot)
   int fo_type, fo_single, fo_ptr, fo_sp;                     // fall-off (by slot)
   int fo_cabr;                                               // 1: chemically activated bimolecular (by slot)
+  // ---- the regions without the packed tables below, which come after them: what the thread-serial kernels stage
+  int base_double, base_int;
+  int warp_int;                                              // ints up to the end of the warp form's (bx_*, fe_*)
   // ---- the reactions once more for the small-mechanism kernels (up to 31 species)
   int rx_dat;                                                // double [nr][4]: lnA, beta, E/R, dnu
   int fg_ent;                                                // double [nnz][2]: signed coefficient, reaction (an int)
@@ -66,8 +69,12 @@ struct MechLayout {
   int bx_order;                                              // int [nr]: fall-off, special forms, third bodies, the rest
   int fe_ent, fe_len;                                        // int [fe_len][nc][2]: entry q of species i's fr list: reaction,
                                                              // high word of the coefficient; fe_len 0: not exact products
-  uint32_t packed_bytes;                                     // of the tables above from rx_dat on
 };
+
+// Bytes of the tables that a kernel stages: the doubles before the packed tables and the first `ints` ints.
+inline constexpr uint32_t staged_bytes(const MechLayout& L, int ints) {
+  return (uint32_t)L.base_double * 8u + (uint32_t)ints * 4u;
+}
 
 // Packed reaction (rx_pack): up to two reactants and two products with coefficient one, or one with two (named
 // twice), an absent second species named nc (concentration 1, g 0), so that the kernels multiply and add without

@@ -236,8 +236,13 @@ void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::
                     const std::vector<int>& fo_slot, const std::vector<int>& plog_slot,
                     const std::vector<int>& cheb_slot, Builder& B, MechLayout& L) {
   const int nc = L.nc, nr = L.nr;
-  const size_t before = B.d.size() * sizeof(double) + B.iv.size() * sizeof(int);
+  while (B.d.size() % 2) B.d.push_back(0.);
+  while (B.iv.size() % 4) B.iv.push_back(0);
+  L.base_double = (int)B.d.size();
+  L.base_int = (int)B.iv.size();
   pack_block(b, rev_kind, tb_slot, fo_slot, plog_slot, cheb_slot, B, L);
+  while (B.iv.size() % 4) B.iv.push_back(0);
+  L.warp_int = (int)B.iv.size();
   std::vector<double> dat(4, 0.), ent(2, 0.);
   std::vector<int> pack(4, 0), order(1, 0), ptr(1, 0);
   L.fg_exact = 1;
@@ -333,7 +338,6 @@ void pack_reactions(const Blob& b, const std::vector<int>& rev_kind, const std::
   L.rx_pack = B.addi(pack);
   L.rx_order = B.addi(order);
   L.fg_ptr = B.addi(ptr);
-  L.packed_bytes = (uint32_t)(B.d.size() * sizeof(double) + B.iv.size() * sizeof(int) - before);
 }
 }  // namespace
 

@@ -25,14 +25,14 @@ __device__ __forceinline__ bool warp_setup(const MechLayout& L, const unsigned c
     warp_mech().gmem = mech_gmem;
     warp_next() = 0;
   }
-  if constexpr (kStaged) return stage_bulk(warp_smem, mech_gmem, L.bytes, &mbar, err);
+  if constexpr (kStaged) return stage_tables(warp_smem, mech_gmem, L, L.warp_int, &mbar, err);
   __syncthreads();
   return true;
 }
 // The warp's work space (in doubles) in the dynamic shared memory
 template <bool kStaged>
 __device__ __forceinline__ int warp_wofs(const MechLayout& L, int ws_doubles) {
-  return (kStaged ? (int)((L.bytes + 15u) / 16u) * 2 : 0) + (int)(threadIdx.x >> 5) * ws_doubles;
+  return (kStaged ? (int)(staged_bytes(L, L.warp_int) / 8u) : 0) + (int)(threadIdx.x >> 5) * ws_doubles;
 }
 // The warp's next cell: a block owns every gridDim-th cell, its warps take them in turn.
 __device__ __forceinline__ long warp_cell() {
@@ -337,13 +337,13 @@ size_t form_bytes(const MechLayout& L, size_t extra) {
   auto even = [](size_t x) { return (x + 1) & ~(size_t)1; };
   const size_t ws = 8 * 32 * 2 + even((size_t)n * (n + 1)) * 2 + 32 * 3 + even(L.nr) * 3 +
                     even(L.n_fo > 0 ? L.n_fo : 1) * 2 + 16 + 6 + extra;
-  return ((L.bytes - L.packed_bytes + 15u) & ~15u) + 4 * ws * sizeof(double);
+  return staged_bytes(L, L.base_int) + 4 * ws * sizeof(double);
 }
 
 // Warps a block, and whether the tables are staged beside their work spaces.  They are unless fewer than four warps
 // would be left, as with some 500 reactions: those read them from global memory.
 int plan_warps(const MechLayout& L, int ws_doubles, bool* staged, size_t* smem) {
-  const size_t mech = (L.bytes + 15u) & ~15u, ws = (size_t)ws_doubles * sizeof(double);
+  const size_t mech = staged_bytes(L, L.warp_int), ws = (size_t)ws_doubles * sizeof(double);
   size_t w = mech < kPlainSmem ? (kPlainSmem - mech) / ws : 0;
   *staged = w >= 4;
   if (!*staged) w = kPlainSmem / ws;

@@ -117,6 +117,17 @@ __device__ __forceinline__ double conc_factor_r(double nu, double c1) {
 
 
 // ---------------------------------------------------------------------------
+// The packed reactions (mech.h rx_pack), read from global memory at block-uniform addresses: staging them would cost
+// the larger mechanisms a block an SM.
+__device__ __forceinline__ const int4*& packed_reactions() {
+  __shared__ const int4* p;
+  return p;
+}
+__device__ __forceinline__ void set_packed_reactions(const MechLayout& L, const unsigned char* mech_gmem) {
+  if (threadIdx.x == 0)
+    packed_reactions() = (const int4*)(mech_gmem + (size_t)L.n_double * sizeof(double) + (size_t)L.rx_pack * sizeof(int));
+}
+
 // Thread-serial RHS of the constant-pressure reactor
 // (BatchReactorHomogeneousConstantPressure.H:175-223).  y: this cell's input
 // vector (stride ns) with component pj replaced by pval when pj >= 0; f: output.
@@ -191,18 +202,22 @@ __device__ __noinline__ double rhs_cell(const MechLayout* __restrict__ Lp, const
   const int* pp = M.I(L.prod_ptr);
   const int* psp = M.I(L.prod_sp);
   const double* pnu = M.D(L.prod_nu);
+  const int4* __restrict__ rx = packed_reactions();
   for (int j = 0; j < NR; ++j) {
     double kArr = exp(lnA[j] + beta[j] * logT - eor[j] * uT);
     if (sgn[j] < 0) kArr *= -1.;
-    if (L.n_plog > 0) {   // pressure-logarithmic reaction (KineticsMap_CHEMKIN.hpp:1341-1348)
+    // the packed form, most reactions': its species by number instead of lists to follow
+    const int4 pk = NC <= 31 ? __ldg(rx + j) : make_int4(0, kRxSpecial, 0, 0);
+    const bool packed = !(pk.y & kRxSpecial);
+    if (!packed && L.n_plog > 0) {   // pressure-logarithmic reaction (KineticsMap_CHEMKIN.hpp:1341-1348)
       const int ps = M.I(L.plog_slot)[j];
       if (ps >= 0) kArr = plog_k(M, L, ps, T, logT, Pk);
     }
-    if (L.n_cheb > 0) {   // Chebyshev reaction (KineticsMap_CHEMKIN.hpp:1332-1339)
+    if (!packed && L.n_cheb > 0) {   // Chebyshev reaction (KineticsMap_CHEMKIN.hpp:1332-1339)
       const int cs = M.I(L.cheb_slot)[j];
       if (cs >= 0) kArr = cheb_k(M, L, cs, T, Pk);
     }
-    if (L.n_xplog > 0) {  // extended PLOG (KineticsMap_CHEMKIN.hpp:1662-1670)
+    if (!packed && L.n_xplog > 0) {  // extended PLOG (KineticsMap_CHEMKIN.hpp:1662-1670)
       const int xs = M.I(L.xplog_slot)[j];
       if (xs >= 0) kArr = xplog_k(M, L, xs, T, logT, Pk, cTotSum, [&](int k) { return SC_(C, k); });
     }
@@ -262,12 +277,43 @@ __device__ __noinline__ double rhs_cell(const MechLayout* __restrict__ Lp, const
       if (cabr) kMod *= (1. / (1. + Pr)) * wF;
       else kMod *= kInf * (Pr / (1. + Pr)) * wF / kArr;
     }
-    if (L.n_xfo > 0) {    // extended fall-off (KineticsMap_CHEMKIN.hpp:1672-1681)
+    if (!packed && L.n_xfo > 0) {    // extended fall-off (KineticsMap_CHEMKIN.hpp:1672-1681)
       const int xs = M.I(L.xfo_slot)[j];
       if (xs >= 0) {
         kArr = xfo_k(M, L, xs, T, cTotSum, [&](int k) { return SC_(C, k); });
         kMod = kArr;
       }
+    }
+    if (packed) {
+      const int s0 = pk.x & 255, s1 = (pk.x >> 8) & 255, p0 = (pk.x >> 16) & 255, p1 = (pk.x >> 24) & 255;
+      double net = SC_(C, s0) * (s1 < NC ? SC_(C, s1) : 1.);
+      if (pk.y & kRxReversible) {
+        double rv = SC_(C, p0) * (p1 < NC ? SC_(C, p1) : 1.);
+        double dg = SC_(G, p0) + (p1 < NC ? SC_(G, p1) : 0.);
+        if (pk.y & kRxTwice) {
+          dg -= SC_(G, s0) + SC_(G, s0);
+        } else {
+          dg -= SC_(G, s0);
+          if (s1 < NC) dg -= SC_(G, s1);
+        }
+        const double rf = exp(dg - lP * dnu[j]);
+        rv *= rf;
+        net -= rv;
+      }
+      net *= kMod;
+      if (pk.y & kRxTwice) {
+        SC_(R, s0) -= net + net;
+      } else {
+        SC_(R, s0) -= net;
+        if (s1 < NC) SC_(R, s1) -= net;
+      }
+      if (p1 == p0) {
+        SC_(R, p0) += net + net;
+      } else {
+        SC_(R, p0) += net;
+        if (p1 < NC) SC_(R, p1) += net;
+      }
+      continue;
     }
     double fwd = 1.;
     for (int q = op[j]; q < op[j + 1]; ++q) fwd *= conc_factor_r(onu[q], SC_(C, osp[q]));
@@ -930,10 +976,11 @@ __global__ void __launch_bounds__(kRT, 4) rounds_rhs_kernel(MechLayout Lp, const
     if (threadIdx.x < kBins + 1) B.bcnt[threadIdx.x] = 0;
     else B.bcur[threadIdx.x - kBins - 1] = 0;
   }
-  if (!stage_bulk(smem, mech_gmem, Lp.bytes, &mbar, err)) return;
+  set_packed_reactions(Lp, mech_gmem);
+  if (!stage_tables(smem, mech_gmem, Lp, Lp.base_int, &mbar, err)) return;
   const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)Lp.n_double * sizeof(double));
-  double* scratch = (double*)(smem + ((Lp.bytes + 15u) & ~15u));
+  const int* Mi = (const int*)(smem + (size_t)Lp.base_double * sizeof(double));
+  double* scratch = (double*)(smem + staged_bytes(Lp, Lp.base_int));
   const RecLayout RL = B.L;
   const int nact = B.nact[par];
   const int njac = B.njac[par];
@@ -1025,10 +1072,11 @@ __global__ void __launch_bounds__(kRT, 4) steady_sources_kernel(MechLayout Lp, c
   __shared__ __align__(8) uint64_t mbar;
   __shared__ MechLayout sL;
   if (threadIdx.x == 0) sL = Lp;
-  if (!stage_bulk(smem, mech_gmem, Lp.bytes, &mbar, err)) return;
+  set_packed_reactions(Lp, mech_gmem);
+  if (!stage_tables(smem, mech_gmem, Lp, Lp.base_int, &mbar, err)) return;
   const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)Lp.n_double * sizeof(double));
-  double* scratch = (double*)(smem + ((Lp.bytes + 15u) & ~15u));
+  const int* Mi = (const int*)(smem + (size_t)Lp.base_double * sizeof(double));
+  double* scratch = (double*)(smem + staged_bytes(Lp, Lp.base_int));
   const int NC = Lp.nc, n = NC + 1;
   const double ZERO_DER = sqrt(kTinyFloat);
   const double ETA2 = sqrt(kMachEpsDouble);
@@ -1318,7 +1366,17 @@ __device__ __noinline__ void steady_sparse_diagonal(const MechLayout* __restrict
 
 // sparseJacobian true: the species diagonal of steady_sparse_diagonal (with speciesEquations on, else
 // zero) and the temperature entry by the forward difference of the dense path (with energyEquation on,
-// else zero).  yb, s0, sp: scratch [n][ncells].
+// else zero).  A block takes 128 cells' source terms, their source terms at the incremented temperature or
+// their diagonal (kind 0, 1, 2): a thread's dependent chain bounds the kernel, and the three are independent,
+// so apart they take less time where the SMs are not full (CH4, 1000 cells: 996 to 693 us) and fill the last wave
+// better where they are (H2/CO, 80 000 cells: 572 to 529 us).  yb, s0, sp: scratch [n][ncells]; kind 1 keeps its state in Sexp.
+__device__ __forceinline__ double steady_t_increment(double yk) {   // linearModel.H:195-230, for the T entry
+  const double ew = 1. / (1.e-12 + 1.e-7 * fabs(yk));
+  double hJ = sqrt(kMachEpsDouble) * fabs(fmax(yk, 1. / ew));
+  hJ = fmax(hJ, 1. / ew);
+  hJ = fmax(hJ, sqrt(kTinyFloat));
+  return fmin(hJ, 1.e-3 + 1e-3 * fabs(yk));
+}
 __global__ void __launch_bounds__(kRT, 4) steady_sources_sparse_kernel(
     MechLayout Lp, const unsigned char* __restrict__ mech_gmem, long ncells, const double* __restrict__ Y,
     const double* __restrict__ T, long ld, const double* __restrict__ pc, double p_scalar, int species, int energy,
@@ -1328,38 +1386,53 @@ __global__ void __launch_bounds__(kRT, 4) steady_sources_sparse_kernel(
   __shared__ __align__(8) uint64_t mbar;
   __shared__ MechLayout sL;
   if (threadIdx.x == 0) sL = Lp;
-  if (!stage_bulk(smem, mech_gmem, Lp.bytes, &mbar, err)) return;
+  set_packed_reactions(Lp, mech_gmem);
+  if (!stage_tables(smem, mech_gmem, Lp, Lp.base_int, &mbar, err)) return;
   const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)Lp.n_double * sizeof(double));
-  double* scratch = (double*)(smem + ((Lp.bytes + 15u) & ~15u));
-  const int NC = Lp.nc, n = NC + 1;
-  for (long c = (long)blockIdx.x * kRT + threadIdx.x; c < ncells; c += (long)gridDim.x * kRT) {
-    for (int i = 0; i < NC; ++i) yb[(long)i * ncells + c] = fmax(Y[(long)i * ld + c], 0.);
-    yb[(long)NC * ncells + c] = T[c];
+  const int* Mi = (const int*)(smem + (size_t)Lp.base_double * sizeof(double));
+  double* scratch = (double*)(smem + staged_bytes(Lp, Lp.base_int));
+  const int NC = Lp.nc;
+  const long chunks = (ncells + kRT - 1) / kRT;
+  for (long it = blockIdx.x; it < 3 * chunks; it += gridDim.x) {
+    const int kind = (int)(it % 3);
+    const long c = it / 3 * kRT + threadIdx.x;
+    if (c >= ncells) continue;
     const double P0 = pc ? pc[c] : p_scalar;
-    const double* y = yb + c;
-    s0[(long)NC * ncells + c] = rhs_cell<true>(&sL, Md, Mi, scratch, y, ncells, -1, 0., s0 + c, ncells, P0, 1, 0.);
-    double JT = 0.;
-    if (energy) {   // linearModel.H:195-230, the dense path's increment for the T entry
-      const double yk = T[c];
-      const double ew = 1. / (1.e-12 + 1.e-7 * fabs(yk));
-      double hJ = sqrt(kMachEpsDouble) * fabs(fmax(yk, 1. / ew));
-      hJ = fmax(hJ, 1. / ew);
-      hJ = fmax(hJ, sqrt(kTinyFloat));
-      const double dy = fmin(hJ, 1.e-3 + 1e-3 * fabs(yk));
-      const double qp = rhs_cell<true>(&sL, Md, Mi, scratch, y, ncells, NC, yk + dy, sp + c, ncells, P0, 1, 0.);
-      JT = (qp - s0[(long)NC * ncells + c]) * (1. / dy);
+    if (kind == 2) {
+      if (species) steady_sparse_diagonal(&sL, Md, Mi, scratch, Y + c, ld, T[c], P0, Simp + c, lds);
+      else
+        for (int k = 0; k < NC; ++k) Simp[(long)k * lds + c] = 0.;
+      continue;
     }
-    if (species) {
-      steady_sparse_diagonal(&sL, Md, Mi, scratch, Y + c, ld, T[c], P0, Simp + c, lds);
+    if (kind == 1 && !energy) continue;
+    double* const y = (kind ? Sexp : yb) + c;
+    double* const f = (kind ? sp : s0) + c;
+    const long ys = kind ? lds : ncells;
+    for (int i = 0; i < NC; ++i) y[(long)i * ys] = fmax(Y[(long)i * ld + c], 0.);
+    y[(long)NC * ys] = T[c];
+    const double q = rhs_cell<true>(&sL, Md, Mi, scratch, y, ys, kind ? NC : -1, T[c] + steady_t_increment(T[c]), f,
+                                    ncells, P0, 1, 0.);
+    f[(long)NC * ncells] = q;
+  }
+}
+// The temperature entry from kinds 0 and 1, and the explicit part of component blockIdx.y.
+__global__ void __launch_bounds__(256) steady_sources_combine_kernel(
+    int NC, long ncells, const double* __restrict__ Y, const double* __restrict__ T, long ld, int energy,
+    const double* __restrict__ s0, const double* __restrict__ sp, double* __restrict__ Simp, double* __restrict__ Sexp,
+    long lds) {
+  const int k = blockIdx.y;
+  for (long c = (long)blockIdx.x * 256 + threadIdx.x; c < ncells; c += (long)gridDim.x * 256) {
+    const double s = s0[(long)k * ncells + c];
+    double J, yk;
+    if (k < NC) {
+      J = Simp[(long)k * lds + c];
+      yk = Y[(long)k * ld + c];
     } else {
-      for (int k = 0; k < NC; ++k) Simp[(long)k * lds + c] = 0.;
+      yk = T[c];
+      J = energy ? (sp[(long)k * ncells + c] - s) * (1. / steady_t_increment(yk)) : 0.;
+      Simp[(long)k * lds + c] = J;
     }
-    Simp[(long)NC * lds + c] = JT;
-    for (int k = 0; k < n; ++k) {
-      const double yk = k < NC ? Y[(long)k * ld + c] : T[c];
-      Sexp[(long)k * lds + c] = s0[(long)k * ncells + c] - Simp[(long)k * lds + c] * yk;
-    }
+    Sexp[(long)k * lds + c] = s - J * yk;
   }
 }
 
@@ -2096,7 +2169,7 @@ cudaError_t launch_steady_sources(const MechLayout& L, const unsigned char* mech
                                   const double* T, long ld, const double* p, double p_scalar, double* scratch,
                                   double* Simp, double* Sexp, long lds, int sm_count, int* err, cudaStream_t stream) {
   if (ncells <= 0) return cudaSuccess;
-  const size_t smem = ((L.bytes + 15u) & ~15u) + (size_t)3 * L.nc * kRT * sizeof(double);
+  const size_t smem = staged_bytes(L, L.base_int) + (size_t)3 * L.nc * kRT * sizeof(double);
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(steady_sources_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -2125,10 +2198,11 @@ __global__ void __launch_bounds__(kRT) jacobian_kernel(MechLayout Lp, const unsi
   __shared__ __align__(8) uint64_t mbar;
   __shared__ MechLayout sL;
   if (threadIdx.x == 0) sL = Lp;
-  if (!stage_bulk(smem, mech_gmem, Lp.bytes, &mbar, err)) return;
+  set_packed_reactions(Lp, mech_gmem);
+  if (!stage_tables(smem, mech_gmem, Lp, Lp.base_int, &mbar, err)) return;
   const double* Md = (const double*)smem;
-  const int* Mi = (const int*)(smem + (size_t)Lp.n_double * sizeof(double));
-  double* scratch = (double*)(smem + ((Lp.bytes + 15u) & ~15u));
+  const int* Mi = (const int*)(smem + (size_t)Lp.base_double * sizeof(double));
+  double* scratch = (double*)(smem + staged_bytes(Lp, Lp.base_int));
   const int n = Lp.nc + 1;
   for (long cell = (long)blockIdx.x * kRT + threadIdx.x; cell < ncells; cell += (long)gridDim.x * kRT) {
     double* Jc = J + cell * (long)n * n;
@@ -2147,7 +2221,7 @@ cudaError_t launch_jacobian(const MechLayout& L, const unsigned char* mech_gmem,
                             double p, int energy, double* J, int sm_count, int* err, cudaStream_t stream) {
   if (ncells <= 0) return cudaSuccess;
   if (L.nc + 1 > 32) return cudaErrorInvalidValue;
-  const size_t smem = ((L.bytes + 15u) & ~15u) + (size_t)3 * L.nc * kRT * sizeof(double);
+  const size_t smem = staged_bytes(L, L.base_int) + (size_t)3 * L.nc * kRT * sizeof(double);
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(jacobian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -2162,7 +2236,7 @@ cudaError_t launch_steady_sources_sparse(const MechLayout& L, const unsigned cha
                                          int species, int energy, double* scratch, double* Simp, double* Sexp,
                                          long lds, int sm_count, int* err, cudaStream_t stream) {
   if (ncells <= 0) return cudaSuccess;
-  const size_t smem = ((L.bytes + 15u) & ~15u) + (size_t)3 * L.nc * kRT * sizeof(double);
+  const size_t smem = staged_bytes(L, L.base_int) + (size_t)3 * L.nc * kRT * sizeof(double);
   if (smem > 227 * 1024) return cudaErrorInvalidValue;
   cudaError_t e =
       cudaFuncSetAttribute(steady_sources_sparse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -2171,11 +2245,16 @@ cudaError_t launch_steady_sources_sparse(const MechLayout& L, const unsigned cha
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, steady_sources_sparse_kernel, kRT, smem);
   if (e != cudaSuccess) return e;
   if (bps <= 0) return cudaErrorInvalidConfiguration;
-  const long want = (ncells + kRT - 1) / kRT, cap = (long)sm_count * bps;
+  const long want = 3 * ((ncells + kRT - 1) / kRT), cap = (long)sm_count * bps;
   const long n = L.nc + 1;
   steady_sources_sparse_kernel<<<(unsigned)(want < cap ? want : cap), kRT, smem, stream>>>(
       L, mech_gmem, ncells, Y, T, ld, p, p_scalar, species, energy, scratch, scratch + n * ncells,
       scratch + 2 * n * ncells, Simp, Sexp, lds, err);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  const long cells256 = (ncells + 255) / 256;
+  const dim3 grid((unsigned)(cells256 < 4096 ? cells256 : 4096), (unsigned)n);
+  steady_sources_combine_kernel<<<grid, 256, 0, stream>>>(L.nc, ncells, Y, T, ld, energy, scratch + n * ncells,
+                                                          scratch + 2 * n * ncells, Simp, Sexp, lds);
   return cudaGetLastError();
 }
 
@@ -2193,7 +2272,7 @@ cudaError_t rounds_prepare(const MechLayout& L, bool lu64, int sm_count, int wid
   *P = RoundsPlan{};
   P->lu64 = lu64;
   P->w = width;
-  P->rhs_smem = ((L.bytes + 15u) & ~15u) + (size_t)3 * L.nc * kRT * sizeof(double);
+  P->rhs_smem = staged_bytes(L, L.base_int) + (size_t)3 * L.nc * kRT * sizeof(double);
   P->adv_smem = advance_smem(L, lu64, width);
   cudaError_t e = cudaFuncSetAttribute(rounds_rhs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)P->rhs_smem);

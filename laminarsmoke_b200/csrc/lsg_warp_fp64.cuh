@@ -43,7 +43,7 @@ __device__ __forceinline__ MechPlace& warp_mech() {
 template <bool kStaged>
 __device__ __forceinline__ MechView warp_tables(const MechLayout& L) {
   const unsigned char* base = kStaged ? (const unsigned char*)warp_smem : warp_mech().gmem;
-  return MechView{(const double*)base, (const int*)(base + (size_t)L.n_double * sizeof(double))};
+  return MechView{(const double*)base, (const int*)(base + (size_t)(kStaged ? L.base_double : L.n_double) * sizeof(double))};
 }
 
 // Per-warp shared-memory workspace (all arrays lane- or index-addressed).
