@@ -9,8 +9,9 @@
 namespace lsg {
 namespace {
 
-// Up to 16 warps a block, one block an SM: 128 registers a thread without spills, the mechanism once per SM.
-constexpr int kPlainWarps = 16;
+// One block an SM, which shares the staged mechanism: up to 16 warps of 128 registers, or up to 8 of 255, whose solver
+// keeps its state in registers (plan_warps).
+constexpr int kPlainWarps = 16, kPlainFew = 8;
 
 // Layout, tables and the block's cell counter; false after a staging time-out.
 __device__ __forceinline__ int& warp_next() {
@@ -45,8 +46,8 @@ __device__ __forceinline__ long warp_cell() {
 // solvers/laminarSMOKE/unsteady/chemistry_DI.H:92-235: gather, clip and
 // renormalise, integrate, renormalise, scatter; Q is the reactor's QR after
 // the solve (chemistry_DI.H:168).
-template <bool kStaged>
-__global__ void __launch_bounds__(kPlainWarps * 32, 1)
+template <bool kStaged, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, 1)
 plain_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepOptions o, StepArgs a,
                   int* err) {
   if (!warp_setup<kStaged>(L, mech_gmem, err)) return;
@@ -148,8 +149,8 @@ __global__ void drg_eps_kernel(long ncells, const double* __restrict__ T, DrgArg
   }
 }
 
-template <bool kStaged>
-__global__ void __launch_bounds__(kPlainWarps * 32, 1)
+template <bool kStaged, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, 1)
 drg_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepOptions o, StepArgs a, DrgArgs d,
                 int* err) {
   if (!warp_setup<kStaged>(L, mech_gmem, err)) return;
@@ -303,8 +304,8 @@ drg_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, StepO
 }
 
 // Standalone right-hand side, one warp per state (same arithmetic as inside the step).
-template <bool kStaged>
-__global__ void __launch_bounds__(kPlainWarps * 32, 1)
+template <bool kStaged, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, 1)
 rhs_warp_kernel(MechLayout L, const unsigned char* __restrict__ mech_gmem, long ncells, const double* __restrict__ y,
                 double* __restrict__ dy, long ld, double p, int energy, double* qr, int* err) {
   if (!warp_setup<kStaged>(L, mech_gmem, err)) return;
@@ -342,33 +343,42 @@ size_t form_bytes(const MechLayout& L, size_t extra) {
 
 // Warps a block, and whether the tables are staged beside their work spaces.  They are unless fewer than four warps
 // would be left, as with some 500 reactions: those read them from global memory.
-int plan_warps(const MechLayout& L, int ws_doubles, bool* staged, size_t* smem) {
+int plan_warps(const MechLayout& L, int ws_doubles, bool* staged, size_t* smem, long cells_per_sm) {
   const size_t mech = staged_bytes(L, L.warp_int), ws = (size_t)ws_doubles * sizeof(double);
   size_t w = mech < kPlainSmem ? (kPlainSmem - mech) / ws : 0;
   *staged = w >= 4;
   if (!*staged) w = kPlainSmem / ws;
   if (w > (size_t)kPlainWarps) w = kPlainWarps;
+  if (w > (size_t)cells_per_sm) w = (size_t)cells_per_sm;
   *smem = (*staged ? mech : 0) + w * ws;
   return (int)w;
 }
 
+// One block an SM, a small batch a cell an SM.  Where no more than 8 warps fit or have a cell, the kernel of 8, which
+// does not spill: CH4, 300 cells 14.5 to 12.2 ms, H2/CO, 67 cells 8.7 to 7.5 ms; with more cells the warps count, H2/CO, 4096 cells
+// 26.1 ms at 16 and 27.0 at 12.
 template <typename K, typename... A>
-cudaError_t launch_warps(const MechLayout& L, int ws_doubles, long ncells, K* staged_kernel, K* global_kernel,
+cudaError_t launch_warps(const MechLayout& L, int ws_doubles, long ncells, K* const (&kernels)[2][2],
                          cudaStream_t stream, A... args) {
-  bool staged = false;
-  size_t smem = 0;
-  const int warps = plan_warps(L, ws_doubles, &staged, &smem);
-  if (warps < 1) return cudaErrorInvalidValue;
-  K* k = staged ? staged_kernel : global_kernel;
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  const long blocks = ncells < sms ? ncells : sms;   // one an SM: a small batch is a cell an SM
+  const long blocks = ncells < sms ? ncells : sms;
+  if (blocks <= 0) return cudaErrorInvalidConfiguration;
+  bool staged = false;
+  size_t smem = 0;
+  const int warps = plan_warps(L, ws_doubles, &staged, &smem, (ncells + blocks - 1) / blocks);
+  if (warps < 1) return cudaErrorInvalidValue;
+  K* k = kernels[staged ? 1 : 0][warps <= kPlainFew ? 0 : 1];
+  if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
   k<<<(unsigned)blocks, warps * 32, smem, stream>>>(args...);
   return cudaGetLastError();
 }
+#define LSG_WARP_KERNELS(k)                                       \
+  {                                                               \
+    {k<false, kPlainFew>, k<false, kPlainWarps>}, { k<true, kPlainFew>, k<true, kPlainWarps> } \
+  }
 }  // namespace
 
 size_t plain_smem_bytes(const MechLayout& L) { return form_bytes(L, 0); }
@@ -378,8 +388,9 @@ size_t drg_smem_bytes(const MechLayout& L) { return form_bytes(L, (size_t)((L.nr
 cudaError_t launch_rhs_warp(const MechLayout& L, const unsigned char* mech_gmem, long ncells, const double* y,
                             double* dy, long ld, double p, int energy, double* qr, int* err, cudaStream_t stream) {
   if (plain_smem_bytes(L) > 227 * 1024) return cudaErrorInvalidValue;
-  return launch_warps(L, warp_ws_doubles(L), ncells, rhs_warp_kernel<true>, rhs_warp_kernel<false>, stream, L,
-                      mech_gmem, ncells, y, dy, ld, p, energy, qr, err);
+  using K = decltype(rhs_warp_kernel<true, kPlainFew>);
+  static K* const kernels[2][2] = LSG_WARP_KERNELS(rhs_warp_kernel);
+  return launch_warps<K>(L, warp_ws_doubles(L), ncells, kernels, stream, L, mech_gmem, ncells, y, dy, ld, p, energy, qr, err);
 }
 
 cudaError_t upload_gear_plain(const GearConsts& gc) {
@@ -389,8 +400,9 @@ cudaError_t upload_gear_plain(const GearConsts& gc) {
 cudaError_t launch_plain(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o,
                          const StepArgs& a, int* err, cudaStream_t stream) {
   if (a.ncells <= 0) return cudaSuccess;
-  return launch_warps(L, warp_ws_doubles(L), a.ncells, plain_warp_kernel<true>, plain_warp_kernel<false>, stream, L,
-                      mech_gmem, o, a, err);
+  using K = decltype(plain_warp_kernel<true, kPlainFew>);
+  static K* const kernels[2][2] = LSG_WARP_KERNELS(plain_warp_kernel);
+  return launch_warps<K>(L, warp_ws_doubles(L), a.ncells, kernels, stream, L, mech_gmem, o, a, err);
 }
 
 cudaError_t launch_drg_eps(long ncells, const double* T, const DrgArgs& d, cudaStream_t stream) {
@@ -404,8 +416,9 @@ cudaError_t launch_drg_plain(const MechLayout& L, const unsigned char* mech_gmem
   if (a.ncells <= 0) return cudaSuccess;
   const cudaError_t e = launch_drg_eps(a.ncells, a.T, d, stream);
   if (e != cudaSuccess) return e;
-  return launch_warps(L, drg_ws_doubles(L), a.ncells, drg_warp_kernel<true>, drg_warp_kernel<false>, stream, L,
-                      mech_gmem, o, a, d, err);
+  using K = decltype(drg_warp_kernel<true, kPlainFew>);
+  static K* const kernels[2][2] = LSG_WARP_KERNELS(drg_warp_kernel);
+  return launch_warps<K>(L, drg_ws_doubles(L), a.ncells, kernels, stream, L, mech_gmem, o, a, d, err);
 }
 
 }  // namespace lsg
