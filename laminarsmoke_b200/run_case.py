@@ -8,9 +8,9 @@ mixtures of H2/CO fuel and air with radicals), h2co_uneven (cold / igniting /
 near-equilibrium thirds; the pool is prepared with the plain step), coflow (the
 200 x 400 Burke-Schumann coflow mesh with H2/CO fuel, 80,000 cells, advanced by
 --steps successive device-resident steps; --cells below 80,000 takes an evenly
-strided subset).  Forms: plain (warp-per-cell FP64), mixed (round scheme, FP32
-factors), batched64 (round scheme, FP64 factors), persistent (persistent lane
-kernel, FP32 factors), group / group64 (fused lane-group kernel, FP32 / FP64
+strided subset).  Forms: plain (warp-per-cell FP64), mixed (batched, FP32
+factors), batched64 (batched, FP64 factors), persistent (persistent lane
+kernel, FP32 factors), group / group64 (resident kernel, FP32 / FP64
 factors), auto (the library's choice: the autotuner for up to 31 species, the
 block-per-cell form above).  --mech h2co+K pads the H2/CO chemistry
 with K inert species (h2co+106: 121 species).
