@@ -54,7 +54,9 @@ extern "C" {
                                   the live cells; the same results either way */
 #define LSG_TILE_PERSISTENT 3  /* one thread per cell, one persistent kernel + device work queue */
 #define LSG_TILE_BLOCK 4       /* one thread block per cell (any size up to 511 species) */
-#define LSG_TILE_GROUP 5       /* the batched form's resident kernel, called asynchronously (up to 31 species) */
+#define LSG_TILE_GROUP 5       /* the batched form's resident kernel, called asynchronously (up to 31 species); where
+                                  no cell fits a block (15 species with 700 reactions), its rounds, which wait for the
+                                  step, or under stream capture the block form */
 /* Mechanisms of 32 to 511 species always run one thread block per cell (the
  * tile is ignored).  The block form factorises in FP64 with LSG_PRECISION_FP64.
  * With LSG_PRECISION_MIXED it inverts G = I - h r0 J on the tensor cores in

@@ -252,11 +252,14 @@ int rhs_dispatch(lsg_ctx* c, long ncells, const double* y, double* dy, long ld, 
   return LSG_OK;
 }
 
+// Lanes a cell of the batched form: the autotuner's, else 0 (by the number of components).
+int tuned_width(const lsg_ctx* c) { return c->tuned && c->tuned_tile == LSG_TILE_LANE ? c->tuned_w : 0; }
+
 int ensure_rounds(lsg_ctx* c, long n, bool lu64) {
   const MechLayout& L = c->mech->host.layout;
   if (L.nc + 1 > 32) return LSG_ERR_UNSUPPORTED;
   if (!sm_count(c)) return LSG_ERR_CUDA;
-  const int w = c->tuned ? c->tuned_w : 0;
+  const int w = tuned_width(c);
   if (c->rplan_lu64 != (int)lu64 || c->rplan_w != w) {
     if (rounds_prepare(L, lu64, c->sm_count, w, &c->rplan) != cudaSuccess) {
       cudaGetLastError();
@@ -404,10 +407,13 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
     const Cand cd = cands[k];
     if (cd.tile == LSG_TILE_LANE && cd.w == 16 && n > 16) continue;
     if (cd.tile == LSG_TILE_WARP && c->opt.precision != LSG_PRECISION_FP64) continue;
+    if (cd.tile == LSG_TILE_GROUP && !resident_fits(L)) continue;   // it would run the rounds
     c->tuned = cd.tile == LSG_TILE_LANE || cd.tile == LSG_TILE_GROUP;
+    c->tuned_tile = cd.tile;
     c->tuned_w = cd.w;
     float ms = 0.f;
-    for (int rep = 0; rep < 2; ++rep) {   // a 1024-cell run pays the one-time set-up, then the timed run
+    bool fits = true;
+    for (int rep = 0; rep < 2 && fits; ++rep) {   // a 1024-cell run pays the one-time set-up, then the timed run
       if (cudaMemcpyAsync(work, pristine, per * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
         c->timer.on = timing;
         return LSG_ERR_CUDA;
@@ -417,7 +423,8 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
       cudaEventRecord(e0, s);
       const int r = launch_tile(c, tr, s, cd.tile);
       cudaEventRecord(e1, s);
-      if (r != LSG_OK || cudaEventSynchronize(e1) != cudaSuccess) {
+      fits = r != LSG_ERR_UNSUPPORTED;   // a form that this mechanism does not fit is not tried
+      if ((r != LSG_OK && fits) || cudaEventSynchronize(e1) != cudaSuccess) {
         c->timer.on = timing;
         c->tuned = false;
         cudaEventDestroy(e0);
@@ -426,14 +433,18 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
       }
       cudaEventElapsedTime(&ms, e0, e1);
     }
+    if (!fits) {
+      cudaGetLastError();
+      continue;
+    }
     c->tune_rate[k] = ms > 0.f ? m / (ms * 1e-3) : 0.;
     if (c->tune_rate[k] > best) { best = c->tune_rate[k]; besti = k; }
   }
   c->timer.on = timing;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
+  c->tuned = besti >= 0;
   if (besti < 0) return LSG_ERR_UNSUPPORTED;
-  c->tuned = true;
   c->tuned_tile = cands[besti].tile;
   c->tuned_w = cands[besti].w;
   return LSG_OK;
@@ -520,12 +531,24 @@ int launch_resident(lsg_ctx* c, const StepArgs& a, const StepOptions& so, int wi
 
 int launch_tile(lsg_ctx* c, const StepArgs& a, cudaStream_t s, int tile) {
   const MechLayout& L = c->mech->host.layout;
-  const StepOptions so = to_step_options(c->opt);
+  StepOptions so = to_step_options(c->opt);
   if (L.nc + 1 > 32 || tile == LSG_TILE_BLOCK) return launch_large(c, a, s);
-  if (tile == LSG_TILE_GROUP && !resident_fits(L)) tile = LSG_TILE_LANE;   // the same solver in rounds
+  if (tile == LSG_TILE_GROUP && !resident_fits(L)) {
+    // the same solver, with the differences that this tile takes, in rounds; these wait for the host, so a call that
+    // is being captured runs the block form, which only enqueues and takes any number of reactions.  Its buffers are
+    // made by the first call, as the resident kernel's queue is.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool captured = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusActive;
+    cudaGetLastError();
+    if (captured) return launch_large(c, a, s);
+    const int r = ensure_block(c);
+    if (r != LSG_OK) return r;
+    tile = LSG_TILE_LANE;
+    so.jacobian = LSG_JACOBIAN_FD;
+  }
   if (tile == LSG_TILE_LANE) {
     const bool lu64 = c->opt.precision == LSG_PRECISION_FP64;
-    const int width = c->tuned ? c->tuned_w : 0;
+    const int width = tuned_width(c);
     if (!sm_count(c)) return LSG_ERR_CUDA;
     if (resident_applies(L, so, a.ncells, width, c->sm_count)) {
       const int r = launch_resident(c, a, so, width, s);
@@ -910,8 +933,8 @@ int lsg_reaction_step_sequence_device(lsg_ctx* c, int nsteps, int ncells, int ns
   }
   int tile = (c->tuned && c->opt.tile == LSG_TILE_AUTO) ? c->tuned_tile : resolve_tile(c->opt);
   if (L.nc + 1 > 32) tile = LSG_TILE_BLOCK;
-  if (tile == LSG_TILE_GROUP && !resident_fits(L)) tile = LSG_TILE_LANE;
-  if (tile == LSG_TILE_LANE) {   // the call waits for each step: no graph
+  // the call waits for each step: no graph
+  if (tile == LSG_TILE_LANE || (tile == LSG_TILE_GROUP && !resident_fits(L))) {
     for (int k = 0; k < nsteps; ++k) {
       a.t0 = t0 + k * dt;
       const int r = launch_tile(c, a, s, tile);
