@@ -138,9 +138,9 @@ def tuning_report(ctx, lsg):
     if t is None:
         return None
     tile, width, rates = t
-    names = {lsg.LSG_TILE_LANE: f"batched form, {width} lanes per cell", lsg.LSG_TILE_WARP: "plain warp kernel",
+    names = {lsg.LSG_TILE_LANE: f"batched form in rounds, {width} lanes per cell", lsg.LSG_TILE_WARP: "plain warp kernel",
              lsg.LSG_TILE_PERSISTENT: "persistent lane kernel",
-             lsg.LSG_TILE_GROUP: "resident kernel, " + ("32 lanes" if width == 2 else "16 lanes") + " per cell",
+             lsg.LSG_TILE_GROUP: "batched form, resident kernel, " + ("32 lanes" if width == 2 else "16 lanes") + " per cell",
              lsg.LSG_TILE_BLOCK: "block per cell, " + ("tensor-core inverse" if width else "FP64 LU factors")}
     return {"chosen": names.get(tile, str(tile)), "sample_cells_per_s": {k: round(v) for k, v in rates.items() if v}}
 

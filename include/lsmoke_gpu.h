@@ -263,12 +263,16 @@ long long lsg_ctx_launches(const lsg_ctx* ctx);
 int lsg_ctx_kernel_times(lsg_ctx* ctx, double* ms, long long* launches, int nkinds, int reset);
 
 /* Result of the autotuner (lsg_options.autotune; no counterpart in the
- * reference): the chosen tile and its variant (lanes per cell, 16 or 32, for
- * the batched form; 4: 16 lanes where the components fit, 2: 32 lanes, for its
- * resident kernel called as LSG_TILE_GROUP; 0 otherwise) and the measured
- * cells/s of the candidates, in the order batched form 16 lanes, batched form
- * 32 lanes, plain warp kernel, persistent lane kernel, resident kernel variants
- * 4 and 2 (0 for a candidate not tried).  For mechanisms above 31 species with
+ * reference): the chosen tile and its variant (LSG_TILE_LANE: the batched
+ * form's rounds with 16 or 32 lanes per cell; LSG_TILE_GROUP: its resident
+ * kernel with 16 (variant 4) or 32 lanes (variant 2); 0 otherwise) and the
+ * measured cells/s of the candidates, in the order rounds 16 lanes, rounds 32
+ * lanes, plain warp kernel, persistent lane kernel, resident kernel 16 lanes,
+ * resident kernel 32 lanes (0 for a candidate not tried).  A tuned context's
+ * calls run either kernel of the batched form as LSG_TILE_LANE does: they wait
+ * for the step, and calls smaller than the trial that the rounds won may run
+ * the resident kernel, with the same results.  With LSG_JACOBIAN_ANALYTIC
+ * only the rounds are tried, which honour it.  For mechanisms above 31 species with
  * LSG_PRECISION_MIXED the candidates are the block form with FP64 LU factors
  * (rates[0]) and with the tensor-core inverse (rates[1]), timed on one wave of
  * the FP64 form's blocks (at least 256 cells); tile is then LSG_TILE_BLOCK and

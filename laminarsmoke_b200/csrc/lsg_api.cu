@@ -63,6 +63,8 @@ struct lsg_ctx {
   // autotuner (lsg_options.autotune)
   bool tuned = false;
   int tuned_tile = 0, tuned_w = 0;
+  int tuned_kernel = 0;         // LSG_TILE_LANE: kTunedRounds or kTunedResident
+  long tuned_cells = 0;         // cells of the trials
   double tune_rate[LSG_NTUNE_CANDIDATES] = {};
   double* tune_buf = nullptr;   // sample cells: pristine copy and work copy
   long tune_cap = 0;
@@ -252,8 +254,20 @@ int rhs_dispatch(lsg_ctx* c, long ncells, const double* y, double* dy, long ld, 
   return LSG_OK;
 }
 
+enum : int { kTunedRounds = 1, kTunedResident = 2 };
+
 // Lanes a cell of the batched form: the autotuner's, else 0 (by the number of components).
 int tuned_width(const lsg_ctx* c) { return c->tuned && c->tuned_tile == LSG_TILE_LANE ? c->tuned_w : 0; }
+
+// Whether the batched form's resident kernel takes a call: by the rule on sizes, unless the autotuner found the
+// resident kernel the faster (which it then is for smaller calls too), or the rounds for a call no larger than this one.
+bool takes_resident(const lsg_ctx* c, const StepOptions& so, long ncells) {
+  if (c->tuned && c->tuned_tile == LSG_TILE_LANE) {
+    if (c->tuned_kernel == kTunedResident) return true;
+    if (ncells >= c->tuned_cells) return false;
+  }
+  return resident_applies(c->mech->host.layout, so, ncells, tuned_width(c), c->sm_count);
+}
 
 int ensure_rounds(lsg_ctx* c, long n, bool lu64) {
   const MechLayout& L = c->mech->host.layout;
@@ -377,9 +391,11 @@ int tune_sample(lsg_ctx* c, const StepArgs& a, cudaStream_t s, long m, StepArgs*
 }
 
 // Autotuner: times the candidate forms on (a copy of) the first cells of the
-// call (up to 262,144) and keeps the fastest for tile LSG_TILE_AUTO.  Candidates: the batched form
-// with 16 lanes a cell (two cells per warp, up to 16 equations) and with 32, the plain warp kernel
-// (FP64 only), the persistent lane kernel and the resident form called directly.
+// call (up to 262,144) and keeps the fastest for tile LSG_TILE_AUTO.  Candidates: the batched form's rounds
+// with 16 lanes a cell (two cells per warp, up to 16 equations) and with 32, the plain warp kernel (FP64 only),
+// the persistent lane kernel and the batched form's resident kernel with 16 and 32 lanes.  Both kernels of the
+// batched form are kept as LSG_TILE_LANE, so whether a tuned call waits for the step does not depend on which won.
+// Where the options ask for the analytic Jacobian and the mechanism has one, only the rounds honour it.
 int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
   const MechLayout& L = c->mech->host.layout;
   const int nc = L.nc, n = nc + 1;
@@ -392,10 +408,12 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
   size_t per = 0;
   const int rs = tune_sample(c, a, s, m, &t, &pristine, &work, &per);
   if (rs != LSG_OK) return rs;
-  struct Cand { int tile, w; };
+  struct Cand { int tile, w, kernel; };
   const Cand cands[LSG_NTUNE_CANDIDATES] = {
-      {LSG_TILE_LANE, 16}, {LSG_TILE_LANE, 32}, {LSG_TILE_WARP, 0}, {LSG_TILE_PERSISTENT, 0},
-      {LSG_TILE_GROUP, 4}, {LSG_TILE_GROUP, 2}};
+      {LSG_TILE_LANE, 16, kTunedRounds},   {LSG_TILE_LANE, 32, kTunedRounds},   {LSG_TILE_WARP, 0, 0},
+      {LSG_TILE_PERSISTENT, 0, 0},         {LSG_TILE_LANE, 16, kTunedResident}, {LSG_TILE_LANE, 32, kTunedResident}};
+  const bool differences = c->opt.jacobian == LSG_JACOBIAN_FD;
+  const bool analytic = !differences && L.n_xplog == 0 && L.n_xfo == 0;
   cudaEvent_t e0, e1;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return LSG_ERR_CUDA;
   double best = -1.;
@@ -407,10 +425,13 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
     const Cand cd = cands[k];
     if (cd.tile == LSG_TILE_LANE && cd.w == 16 && n > 16) continue;
     if (cd.tile == LSG_TILE_WARP && c->opt.precision != LSG_PRECISION_FP64) continue;
-    if (cd.tile == LSG_TILE_GROUP && !resident_fits(L)) continue;   // it would run the rounds
-    c->tuned = cd.tile == LSG_TILE_LANE || cd.tile == LSG_TILE_GROUP;
+    if (cd.kernel == kTunedResident && !(differences && resident_fits(L, cd.w))) continue;
+    if (cd.kernel != kTunedRounds && analytic) continue;
+    c->tuned = cd.tile == LSG_TILE_LANE;
     c->tuned_tile = cd.tile;
     c->tuned_w = cd.w;
+    c->tuned_kernel = cd.kernel;
+    c->tuned_cells = 0;
     float ms = 0.f;
     bool fits = true;
     for (int rep = 0; rep < 2 && fits; ++rep) {   // a 1024-cell run pays the one-time set-up, then the timed run
@@ -447,6 +468,8 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
   if (besti < 0) return LSG_ERR_UNSUPPORTED;
   c->tuned_tile = cands[besti].tile;
   c->tuned_w = cands[besti].w;
+  c->tuned_kernel = cands[besti].kernel;
+  c->tuned_cells = m;
   return LSG_OK;
 }
 
@@ -548,10 +571,9 @@ int launch_tile(lsg_ctx* c, const StepArgs& a, cudaStream_t s, int tile) {
   }
   if (tile == LSG_TILE_LANE) {
     const bool lu64 = c->opt.precision == LSG_PRECISION_FP64;
-    const int width = tuned_width(c);
     if (!sm_count(c)) return LSG_ERR_CUDA;
-    if (resident_applies(L, so, a.ncells, width, c->sm_count)) {
-      const int r = launch_resident(c, a, so, width, s);
+    if (takes_resident(c, so, a.ncells)) {
+      const int r = launch_resident(c, a, so, tuned_width(c), s);
       if (r != LSG_OK) return r;
       // as with the round scheme, the call returns when the step is done
       if (cudaStreamSynchronize(s) != cudaSuccess) return LSG_ERR_CUDA;
@@ -569,8 +591,7 @@ int launch_tile(lsg_ctx* c, const StepArgs& a, cudaStream_t s, int tile) {
   if (tile == LSG_TILE_GROUP) {
     if (L.nc + 1 > 32) return LSG_ERR_UNSUPPORTED;
     if (!sm_count(c)) return LSG_ERR_CUDA;
-    // the autotuner's variant 2: a warp a cell; else 16 lanes where the components fit
-    return launch_resident(c, a, so, (c->tuned && c->tuned_w == 2) ? 32 : 0, s);
+    return launch_resident(c, a, so, 0, s);
   }
   if (tile == LSG_TILE_WARP) {
     if (L.nc + 1 > 32) return LSG_ERR_UNSUPPORTED;
@@ -785,8 +806,10 @@ long long lsg_ctx_launches(const lsg_ctx* c) { return c ? c->launches : -1; }
 
 int lsg_ctx_tuning(const lsg_ctx* c, int* tile, int* width, double* rates) {
   if (!c || !c->tuned || c->opt.tile != LSG_TILE_AUTO || !c->opt.autotune) return LSG_ERR_ARG;
-  if (tile) *tile = c->tuned_tile;
-  if (width) *width = c->tuned_w;
+  // the resident kernel by its own tile and variant
+  const bool resident = c->tuned_tile == LSG_TILE_LANE && c->tuned_kernel == kTunedResident;
+  if (tile) *tile = resident ? LSG_TILE_GROUP : c->tuned_tile;
+  if (width) *width = resident ? (c->tuned_w == 16 ? 4 : 2) : c->tuned_w;
   if (rates)
     for (int k = 0; k < LSG_NTUNE_CANDIDATES; ++k) rates[k] = c->tune_rate[k];
   return LSG_OK;

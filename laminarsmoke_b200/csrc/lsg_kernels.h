@@ -163,7 +163,8 @@ cudaError_t launch_rhs_warp(const MechLayout& L, const unsigned char* mech_gmem,
 // 32 or 0: by the number of components); queue: one int
 cudaError_t launch_group(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o, const StepArgs& a,
                          bool lu64, int width, int* queue, int sm_count, cudaStream_t stream);
-bool resident_fits(const MechLayout& L);   // a block's shared memory holds at least one warp's cells
+// a block's shared memory holds at least one warp's cells, `width` lanes each (0: as launch_group)
+bool resident_fits(const MechLayout& L, int width = 0);
 bool resident_applies(const MechLayout& L, const StepOptions& o, long ncells, int width, int sm_count);
 
 // Jacobians with analytic species columns (lsg_rounds.cu), up to 31 species; J [ncells][n][n] row-major

@@ -2367,7 +2367,10 @@ bool resident_applies(const MechLayout& L, const StepOptions& o, long ncells, in
   return teams >= 8 || ncells <= (long)sm_count * teams * 32;
 }
 
-bool resident_fits(const MechLayout& L) { return L.nc + 1 <= 32 && team_count(L, L.nc + 1 <= 16 ? 16 : 32) > 0; }
+bool resident_fits(const MechLayout& L, int width) {
+  if (width == 0) width = L.nc + 1 <= 16 ? 16 : 32;
+  return L.nc + 1 <= width && team_count(L, width) > 0;
+}
 
 // Resident form on all cells of a call, `width` lanes a cell (0: 16 where the components fit, else 32).
 cudaError_t launch_group(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o, const StepArgs& a,

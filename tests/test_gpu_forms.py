@@ -91,3 +91,42 @@ def test_autotuner_skips_a_form_without_room(cuda, rich, precision):
     if width == 16:   # the lanes of a default call
         for a, b in zip(got, (Yr, Tr, cnt)):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+def test_autotuner_honours_the_analytic_jacobian(cuda, h2co, precision):
+    """A tuned context that asks for the analytic Jacobian integrates with it: one evaluation a Jacobian (its
+    temperature column), whichever form would be the faster with differences."""
+    from laminarsmoke_b200 import lsg
+    data, species, A = h2co
+    Y, T = cells.h2co_mixing(species, A["mw"], 2048, seed=8)
+    import torch
+    Y, T = torch.tensor(np.ascontiguousarray(Y.T), device=cuda), torch.tensor(T, device=cuda)
+    ctx = lsg.ReactionStep(lsg.Mechanism(data), precision=precision, autotune=1, jacobian=lsg.LSG_JACOBIAN_ANALYTIC)
+    cnt = _step(ctx, Y, T, 1e-5)[2]
+    assert cnt[:, 2].sum() > 0 and (cnt[:, 7] == cnt[:, 2]).all()
+    assert {k for k, v in ctx.tuning()[2].items() if v > 0} == {"rounds16", "rounds32"}
+
+
+def test_autotuner_times_each_kernel_once(cuda, h2co):
+    """Rounds and resident kernel are candidates of their own, and a tuned context's step sequences run one by one
+    whichever of the two won, as LSG_TILE_LANE's do."""
+    import torch
+    from laminarsmoke_b200 import lsg
+    data, species, A = h2co
+    Y, T = cells.h2co_mixing(species, A["mw"], 1500, seed=8)
+    Y, T = torch.tensor(np.ascontiguousarray(Y.T), device=cuda), torch.tensor(T, device=cuda)
+    ctx = lsg.ReactionStep(lsg.Mechanism(data), precision=lsg.LSG_PRECISION_MIXED, autotune=1)
+    got = _step(ctx, Y, T, 1e-5)
+    tile, width, rates = ctx.tuning()
+    assert {k for k, v in rates.items() if v > 0} == {"rounds16", "rounds32", "persistent", "group_4", "group_2"}
+    assert ctx.launches() > 1000   # hundreds of rounds of four launches each, for two lane widths
+    if width in (16, 4):
+        want = _step(lsg.ReactionStep(lsg.Mechanism(data), precision=lsg.LSG_PRECISION_MIXED), Y, T, 1e-5)
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
+    Yd, Td = Y.clone(), T.clone()
+    if tile in (lsg.LSG_TILE_LANE, lsg.LSG_TILE_GROUP):
+        assert not ctx.step_sequence_graph(Yd, Td, 1e-5, 2)
+    torch.cuda.synchronize()
+    ctx.check()
