@@ -2414,9 +2414,8 @@ namespace {
 // 45 components 22.0 and 11.4 at 96 cells, 42.5 and 35.4 at 592, 1986 and 1469 at 30 000; 121 components 18.3 and 6.2
 // at one cell, 88.9 and 60.9 at 592, 694 and 485 at 6000; 800 reactions and 121 components 811 and 357 at 96 cells,
 // 1798 and 1377 at 1200.
-bool shared_factors(const MechLayout& L) {
-  return block_sg_bytes<256>(L) + 2048 <= 227 * 1024;   // 2048: static shared memory and the block's reserve
-}
+constexpr size_t kSgSmem = 225 * 1024;   // of 227 KB: the rest for the static shared memory and the block's reserve
+bool shared_factors(const MechLayout& L) { return block_sg_bytes<256>(L) <= kSgSmem; }
 }  // namespace
 
 cudaError_t launch_block(const MechLayout& L, const unsigned char* mech_gmem, const StepOptions& o,
@@ -2441,7 +2440,8 @@ cudaError_t launch_block(const MechLayout& L, const unsigned char* mech_gmem, co
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(block_kernel<kT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the same value at every call: another thread may launch the kernel with another size at the same time
+    e = cudaFuncSetAttribute(block_kernel<kT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSgSmem);
     if (e != cudaSuccess) return e;
     g = g < sms ? g : sms;   // one block an SM (nblocks, the work spaces, is at least the SM count)
     block_kernel<kT, false, true><<<(unsigned)g, kT, smem, stream>>>(L, mech_gmem, o, a, ws, queue, err);

@@ -371,7 +371,9 @@ cudaError_t launch_warps(const MechLayout& L, int ws_doubles, long ncells, K* co
   const int warps = plan_warps(L, ws_doubles, &staged, &smem, (ncells + blocks - 1) / blocks);
   if (warps < 1) return cudaErrorInvalidValue;
   K* k = kernels[staged ? 1 : 0][warps <= kPlainFew ? 0 : 1];
-  if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+  // the same value at every call: another thread may launch the kernel with another size at the same time
+  e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlainSmem);
+  if (e != cudaSuccess) return e;
   k<<<(unsigned)blocks, warps * 32, smem, stream>>>(args...);
   return cudaGetLastError();
 }

@@ -329,8 +329,9 @@ namespace {
 template <int BD, bool STAGED>
 cudaError_t props(const MechLayout& L, const unsigned char* mech_gmem, const TransportLayout& TL,
                   const unsigned char* tr_gmem, const PropArgs& a, size_t smem, cudaStream_t stream) {
-  const cudaError_t e =
-      cudaFuncSetAttribute(properties_kernel<BD, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the same value at every call: another thread may launch the kernel with another size at the same time
+  const cudaError_t e = cudaFuncSetAttribute(properties_kernel<BD, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kPropSmemMax);
   if (e != cudaSuccess) return e;
   const long grid = (a.ncells + BD - 1) / BD;
   properties_kernel<BD, STAGED><<<(unsigned)grid, BD, smem, stream>>>(L, mech_gmem, TL, tr_gmem, a);

@@ -1367,13 +1367,14 @@ __global__ void __launch_bounds__(kTeamThreads, 1)
 
 namespace {
 
+constexpr size_t kTeamSmem = 222 * 1024;   // of 227 KB: the static arrays and the layouts take the rest
+
 // Teams of a block: what the SM's shared memory holds beside the slots, whole warps, at most one per slot and
 // per W threads; 0 when not even one warp's teams fit.
 inline int team_count(const MechLayout& L, int w) {
   const size_t slots = (size_t)slot_layout(L).total * sizeof(double), per = (size_t)team_layout(L.nc + 1).total * sizeof(double);
-  const size_t most = 222 * 1024;   // of 227 KB: the static arrays and the layouts take the rest
-  if (slots + per * (32 / w) > most) return 0;
-  long k = (long)((most - slots) / per);
+  if (slots + per * (32 / w) > kTeamSmem) return 0;
+  long k = (long)((kTeamSmem - slots) / per);
   if (k > kSlots) k = kSlots;
   if (k > kTeamThreads / w) k = kTeamThreads / w;
   return (int)(k - k % (32 / w));
@@ -1388,7 +1389,9 @@ cudaError_t team_launch(const MechLayout& L, const unsigned char* mech_gmem, con
   const long need = (a.ncells + grid - 1) / grid;   // cells a block
   if (need < teams) teams = (int)((need + 32 / W - 1) / (32 / W) * (32 / W));
   const size_t smem = sizeof(double) * ((size_t)slot_layout(L).total + (size_t)teams * team_layout(L.nc + 1).total);
-  cudaError_t e = cudaFuncSetAttribute(team_kernel<LUT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the same value at every call: another thread may launch the kernel with another size at the same time
+  cudaError_t e =
+      cudaFuncSetAttribute(team_kernel<LUT, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTeamSmem);
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(queue, 0, sizeof(int), stream);
   if (e != cudaSuccess) return e;
