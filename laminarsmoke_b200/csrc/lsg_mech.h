@@ -97,7 +97,9 @@ struct TransportLayout {
   int wilke;                  // [nc][nc][2]: sqrt(phi) and sqrt(phi) (M_j / M_k)^(1/4), phi = 1 / sqrt(8 (1 + M_k / M_j))
   // ---- int region
   int iteta;                  // [n_teta] species index of each light species
+  double T_min, T_max;        // between which no fit's exponent exceeds kFitExponent in magnitude (min > max: none)
 };
+constexpr double kFitExponent = 680.;
 
 // Views into a flattened table (global or shared memory).
 struct MechView {

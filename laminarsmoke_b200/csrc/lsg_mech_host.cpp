@@ -78,6 +78,50 @@ struct Builder {
 };
 }  // namespace
 
+// The temperatures around 1000 K at which every row c0 + c1 x + c2 x^2 + c3 x^3, x = ln T, of the fits stays within
+// kFitExponent in magnitude, and the sum of its terms' magnitudes small enough for the rounding of the row not to matter.
+static void fit_range(const std::vector<const std::vector<double>*>& fits, double* lo, double* hi) {
+  auto row_within = [](const double* c, double a, double b) {
+    auto ok = [&](double x) {
+      const double v = c[0] + x * (c[1] + x * (c[2] + x * c[3]));
+      const double s = std::fabs(c[0]) + std::fabs(x) * (std::fabs(c[1]) + std::fabs(x) * (std::fabs(c[2]) + std::fabs(x * c[3])));
+      return std::fabs(v) <= kFitExponent && s <= 1.e12;   // false for NaN
+    };
+    if (!ok(a) || !ok(b)) return false;
+    // between the ends the extremes are where c1 + 2 c2 x + 3 c3 x^2 = 0
+    const double d = c[2] * c[2] - 3. * c[3] * c[1];
+    if (d < 0.) return true;
+    const double q = -(c[2] + std::copysign(std::sqrt(d), c[2]));
+    const double root[2] = {q / (3. * c[3]), c[1] / q};
+    for (double x : root)
+      if (x > a && x < b && !ok(x)) return false;
+    return true;
+  };
+  auto within = [&](double a, double b) {
+    for (const std::vector<double>* f : fits)
+      for (size_t r = 0; r + 4 <= f->size(); r += 4)
+        if (!row_within(f->data() + r, a, b)) return false;
+    return true;
+  };
+  const double mid = std::log(1000.);
+  *lo = 1.;
+  *hi = 0.;
+  if (!within(mid, mid)) return;
+  double a = mid, b = mid;
+  double out = -750.;   // below ln of the smallest positive double
+  for (int i = 0; i < 64; ++i) {
+    const double x = 0.5 * (a + out);
+    (within(x, b) ? a : out) = x;
+  }
+  out = 710.;           // above ln of the largest
+  for (int i = 0; i < 64; ++i) {
+    const double x = 0.5 * (b + out);
+    (within(a, x) ? b : out) = x;
+  }
+  *lo = std::fmax(std::exp(a) * (1. + 1.e-9), 1.e-300);   // kFitExponent is some way below what the kernel can take
+  *hi = std::fmin(std::exp(b) * (1. - 1.e-9), 1.e300);
+}
+
 // The transport fits, when the blob has them, with the Wilke factors of every
 // species pair (TransportPropertiesMap_CHEMKIN.hpp:653-688) precomputed.
 static bool build_transport(const Blob& b, int nc, HostMech& out, std::string& err) {
@@ -118,6 +162,7 @@ static bool build_transport(const Blob& b, int nc, HostMech& out, std::string& e
   T.teta = B.addd(teta.empty() ? std::vector<double>(2, 0.) : teta);
   T.wilke = B.addd(wilke);
   T.iteta = B.addi(it.empty() ? std::vector<int>(1, 0) : it);
+  fit_range({&eta, &lam, &gam}, &T.T_min, &T.T_max);
   while (B.d.size() % 2) B.d.push_back(0.);
   while (B.iv.size() % 4) B.iv.push_back(0);
   T.n_double = (int)B.d.size();

@@ -52,8 +52,8 @@ constexpr double kMu0 = 1.8405e-5, kT0 = 300., kBeta0 = 0.6759, kPr0 = 0.7;   //
 
 // e^x for the fits: x = k ln 2 + r with |r| <= ln 2 / 2 (ln 2 as an unevaluated sum of two doubles) and the Taylor
 // polynomial of degree 13, whose remainder is below 4e-18, without a branch, so that several run interleaved.  It
-// holds for |x| <= 690; `top` collects the high words' magnitudes, and a cell that exceeds the bound (or is NaN
-// somewhere) is evaluated again with the library's exp (kFast false).  The constants are held in registers through
+// holds for |x| <= 690; a cell whose temperature lets a fit's exponent come near that (TransportLayout::T_min: far
+// outside the fits, or NaN) is evaluated with the library's exp (kFast false).  The constants are held in registers through
 // volatile asm: left to itself the compiler rebuilds each with two moves before every use.
 struct ExpConst {
   double c[13];   // 1 / 13!, 1 / 12!, ..., 1 / 3!, then log2(e), ln 2
@@ -64,11 +64,9 @@ struct ExpConst {
     for (int i = 0; i < 13; ++i) asm volatile("mov.f64 %0, %1;" : "=d"(c[i]) : "d"(v[i]));
   }
 };
-constexpr int kExpTop = 0x40859000;   // high word of 690.
 template <bool kFast>
-__device__ __forceinline__ double exp_fit(const ExpConst& e, double x, int& top) {
+__device__ __forceinline__ double exp_fit(const ExpConst& e, double x) {
   if constexpr (!kFast) return exp(x);
-  top = max(top, __double2hiint(x) & 0x7fffffff);
   constexpr double kRound = 6755399441055744.;   // 1.5 * 2^52: adding it rounds to an integer
   const double t = fma(x, e.c[11], kRound), k = t - kRound;
   double r = fma(-k, e.c[12], x);
@@ -127,26 +125,38 @@ struct Tables {
   const int* TI;
 };
 
-// One cell; returns whether a fit's exponent left exp_fit's range.
-template <int BD, bool kFast>
-__device__ __forceinline__ bool cell_properties(const MechLayout& L, const TransportLayout& TL, const PropArgs& a,
-                                                const Tables& tb, double* xs, double* us, long c) {
-  const int nc = L.nc;
-  const double *MD = tb.MD, *TD = tb.TD, *TM = tb.TM;
-  const double* MW = MD + L.mw;
-  const long ld = a.ld, lo = a.ld_out;
-  const ExpConst E;
-  int top = 0;
-  const double T = __ldcs(a.T + c);
-  const double p = a.p ? __ldcs(a.p + c) : a.p_scalar;
+// What a cell reads: its mass fractions go to xs.  All of it is read before anything is written, so that a field may
+// take the place of an input.
+struct CellInputs {
+  double T, p, u;   // temperature, pressure, sum Y_i / MW_i
+};
+template <int BD>
+__device__ __forceinline__ CellInputs cell_inputs(const PropArgs& a, const double* MW, int nc, double* xs, long c) {
+  CellInputs in;
+  in.T = __ldcs(a.T + c);
+  in.p = a.p ? __ldcs(a.p + c) : a.p_scalar;
   double u = 0.;
 #pragma unroll 4
   for (int s = 0; s < nc; ++s) {
-    const double y = __ldcs(a.Y + s * ld + c);
+    const double y = __ldcs(a.Y + s * a.ld + c);
     xs[s * BD] = y;
     u += div_z(y, MW[s]);
   }
-  const double MWm = 1. / u;
+  in.u = u;
+  return in;
+}
+
+// One cell.
+template <int BD, bool kFast>
+__device__ __forceinline__ void cell_properties(const MechLayout& L, const TransportLayout& TL, const PropArgs& a,
+                                                const Tables& tb, double* xs, double* us, long c, const CellInputs& in) {
+  const int nc = L.nc;
+  const double *MD = tb.MD, *TD = tb.TD, *TM = tb.TM;
+  const double* MW = MD + L.mw;
+  const long lo = a.ld_out;
+  const ExpConst E;
+  const double T = in.T, p = in.p;
+  const double MWm = 1. / in.u;
   const double cTot = p / kRgas / T;
   const double psi = cTot * MWm / p;
   if (a.MWmix) __stcs(a.MWmix + c, MWm);
@@ -166,11 +176,11 @@ __device__ __forceinline__ bool cell_properties(const MechLayout& L, const Trans
       hmix += (d[0] + T * d[1] + T2 * d[2] + T3 * d[3] + T4 * d[4] + uT * d[5]) * x;
     }
     const double half = 0.5 * cubic(TD + TL.eta + 4 * s, lT);
-    us[s * BD] = exp_fit<kFast>(E, -half, top);
+    us[s * BD] = exp_fit<kFast>(E, -half);
     if (thermal) {
       const double ll = cubic(TD + TL.lam + 4 * s, lT);
-      l1 = fma(x, exp_fit<kFast>(E, ll, top), l1);
-      l2 = fma(x, exp_fit<kFast>(E, -ll, top), l2);
+      l1 = fma(x, exp_fit<kFast>(E, ll), l1);
+      l2 = fma(x, exp_fit<kFast>(E, -ll), l2);
       const double* q = (hi ? MD + L.cp_ht : MD + L.cp_lt) + 5 * s;
       const double cpr = q[0] + T * q[1] + T2 * q[2] + T3 * q[3] + T4 * q[4];
       cpm += cpr * x;
@@ -215,7 +225,7 @@ __device__ __forceinline__ bool cell_properties(const MechLayout& L, const Trans
   if (a.mu) __stcs(a.mu + c, mu);
   if (thermal && a.lambda) __stcs(a.lambda + c, lambda);
 
-  if (!a.Dmix) return top > kExpTop;
+  if (!a.Dmix) return;
   const int* it = tb.TI;
   if (a.Dsoret) {   // the thermal-diffusion ratios, while x is at hand; scaled by Dmix below
     const double* ft = TD + TL.teta;
@@ -262,7 +272,7 @@ __device__ __forceinline__ bool cell_properties(const MechLayout& L, const Trans
           v[q] = acc[(j + q) * BD];
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) g[q] = exp_fit<kFast>(E, g[q], top);
+        for (int q = 0; q < 4; ++q) g[q] = exp_fit<kFast>(E, g[q]);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           sk = fma(xs[(j + q) * BD], g[q], sk);
@@ -270,7 +280,7 @@ __device__ __forceinline__ bool cell_properties(const MechLayout& L, const Trans
         }
       }
       for (; j < nc; ++j, fg += 4) {
-        const double g = exp_fit<kFast>(E, -cubic(fg, lT), top);
+        const double g = exp_fit<kFast>(E, -cubic(fg, lT));
         sk = fma(xs[j * BD], g, sk);
         acc[j * BD] = fma(xk, g, acc[j * BD]);
       }
@@ -279,19 +289,18 @@ __device__ __forceinline__ bool cell_properties(const MechLayout& L, const Trans
       __stcs(a.Dmix + k * lo + c, D);
     }
   }
-  if (!a.Dsoret) return top > kExpTop;
+  if (!a.Dsoret) return;
   for (int m = 0; m < TL.n_teta; ++m) {
     const int i = it[m];
     a.Dsoret[m * lo + c] = acc[i * BD] * a.Dsoret[m * lo + c] * MW[i] / MWm;
   }
-  return top > kExpTop;
 }
 
 // The same cell with the library's exponentials.
 template <int BD>
 __device__ __noinline__ void cell_properties_slow(const MechLayout& L, const TransportLayout& TL, const PropArgs& a,
-                                                  const Tables& tb, double* xs, double* us, long c) {
-  cell_properties<BD, false>(L, TL, a, tb, xs, us, c);
+                                                  const Tables& tb, double* xs, double* us, long c, const CellInputs in) {
+  cell_properties<BD, false>(L, TL, a, tb, xs, us, c, in);
 }
 
 // BD threads a block; STAGED: the tables are in shared memory (the mechanism's doubles up to the entropy fits and the
@@ -322,7 +331,9 @@ __global__ void __launch_bounds__(BD) properties_kernel(const __grid_constant__ 
   }
   const long c = blockIdx.x * (long)BD + threadIdx.x;
   if (c >= a.ncells) return;   // no block barriers below
-  if (cell_properties<BD, true>(L, TL, a, tb, xs, us, c)) cell_properties_slow<BD>(L, TL, a, tb, xs, us, c);
+  const CellInputs in = cell_inputs<BD>(a, tb.MD + L.mw, nc, xs, c);
+  if (in.T >= TL.T_min && in.T <= TL.T_max) cell_properties<BD, true>(L, TL, a, tb, xs, us, c, in);
+  else cell_properties_slow<BD>(L, TL, a, tb, xs, us, c, in);
 }
 
 namespace {
