@@ -89,7 +89,7 @@ __device__ __forceinline__ double bcast(double v, int src, double* slot) {
 struct BlockShared {
   double* Z;     // [8][BT]
   double* V;     // [8][BT]
-  double* C;     // [NC] concentrations
+  double* C;     // [NC + 1] concentrations, then 1
   double* H;     // [NC] h/RT
   double* S;     // [NC] s/R
   double* NET;   // [NR] net rates
@@ -104,10 +104,33 @@ struct BlockShared {
   unsigned char* DROP = nullptr;  // [NR]
 };
 
+// Doubles for H, S and NET: the enthalpies and entropies are read only while an evaluation renews its kinetic constants,
+// before it writes a rate, so they lie where the rates come to lie.
+__host__ __device__ inline int block_rate_doubles(const MechLayout& L) { return L.nr > 2 * L.nc ? L.nr : 2 * L.nc; }
+
 template <int BT>
 __host__ __device__ inline size_t block_shared_bytes(const MechLayout& L) {
-  return sizeof(double) * (16 * BT + 3 * (size_t)L.nc + 2 + (size_t)L.nr + BT + 2 * (BT / 32) + 4) +
-         sizeof(int) * (2 * BT + BT / 32 + 1) + 64;
+  return sizeof(double) * (16 * BT + (size_t)L.nc + 1 + (size_t)block_rate_doubles(L) + BT + 2 * (BT / 32) + 4) +
+         sizeof(int) * (2 * BT);
+}
+
+// The arrays above from p on; ZS: the stride of the Nordsieck rows.
+template <int BT, int ZS = BT>
+__device__ __forceinline__ BlockShared carve_block(double* p, const MechLayout& L) {
+  BlockShared W;
+  W.X = p; p += BT;
+  W.Z = p; p += 8 * ZS;
+  W.V = p; p += 8 * ZS;
+  W.C = p; p += L.nc + 1;
+  W.NET = W.H = p;
+  W.S = W.H + L.nc;
+  p += block_rate_doubles(L);
+  W.red = p; p += 2 * (BT / 32);
+  W.slot = p; p += 4;
+  W.PIV = (int*)p;
+  W.PERM = W.PIV + BT;
+  W.ival = (int*)(W.red + BT / 32);   // the second half of red: barriers part a sum from a factorisation
+  return W;
 }
 
 // The factors of SG and their work arrays (GearBlock::lu_*), in doubles: G, U, P, R, candidates, flags.
@@ -306,7 +329,6 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
     const double* A = (hi ? M.D(L.dh_ht) : M.D(L.dh_lt)) + 6 * tid;
     hl = A[0] + T * A[1] + T2 * A[2] + T3 * A[3] + T4 * A[4] + uT * A[5];
     C[tid] = cl;
-    H[tid] = hl;
   } else if (tid == NC) {
     C[NC] = 1.;   // the packed reactions' absent second species
   }
@@ -315,6 +337,7 @@ __device__ __noinline__ double rhs_block(const RhsPlace R, const double* __restr
   if (recalc && tid < NC) {
     const double logT = log(T);
     const double* A = (hi ? M.D(L.ds_ht) : M.D(L.ds_lt)) + 6 * tid;
+    H[tid] = hl;
     S[tid] = A[0] * logT + T * A[1] + T2 * A[2] + T3 * A[3] + T4 * A[4] + A[5];
   }
   __syncthreads();
@@ -1828,18 +1851,7 @@ __global__ void __launch_bounds__(BT, SG ? 1 : TC ? (BT == 128 ? 2 : 1) : (BT ==
   } else {
     double* p = (double*)bsm;
     if constexpr (SG) p += shared_lu_doubles(ne);   // the factors come first, then X: 16-byte aligned
-    W.X = p; p += BT;
-    W.Z = p; p += 8 * (SG ? 128 : BT);
-    W.V = p; p += 8 * (SG ? 128 : BT);
-    W.C = p; p += NC + 2;
-    W.H = p; p += NC;
-    W.S = p; p += NC;
-    W.NET = p; p += L.nr;
-    W.red = p; p += 2 * (BT / 32);
-    W.slot = p; p += 4;
-    W.PIV = (int*)p;
-    W.ival = W.PIV + BT;
-    W.PERM = W.ival + BT / 32 + 1;
+    W = carve_block<BT, SG ? 128 : BT>(p, L);
   }
   // mixed-precision form: the tensor-core inverse's operands after the FP64 work space, 1024-byte aligned,
   // then its small arrays; TMEM (256 columns) for the block's lifetime
@@ -1997,22 +2009,7 @@ __global__ void __launch_bounds__(BT, BT == 128 ? 4 : (BT == 256 ? 2 : 1))
   double* Jp = ws;
   double* Gp = ws + (size_t)(NC + 1) * (NC + 1);
   double* karr = ws + 2 * (size_t)(NC + 1) * (NC + 1);
-  BlockShared W;
-  {
-    double* p = (double*)bsm;
-    W.Z = p; p += 8 * BT;
-    W.V = p; p += 8 * BT;
-    W.C = p; p += NC + 2;
-    W.H = p; p += NC;
-    W.S = p; p += NC;
-    W.NET = p; p += L.nr;
-    W.X = p; p += BT;
-    W.red = p; p += 2 * (BT / 32);
-    W.slot = p; p += 4;
-    W.PIV = (int*)p;
-    W.ival = W.PIV + BT;
-    W.PERM = W.ival + BT / 32 + 1;
-  }
+  BlockShared W = carve_block<BT>((double*)bsm, L);
   unsigned char* ex = bsm + ((block_shared_bytes<BT>(L) + 15) & ~(size_t)15);
   W.DX = (double*)ex;
   int* WC = (int*)(W.DX + BT);          // per-warp counts
@@ -2312,22 +2309,7 @@ __global__ void __launch_bounds__(BT) rhs_block_kernel(MechLayout L, const unsig
   double* ukeq = karr + L.nr;
   double* kinf = ukeq + L.nr;
   double* logf = kinf + (L.n_fo > 0 ? L.n_fo : 1);
-  BlockShared W;
-  {
-    double* q = (double*)bsm;
-    W.Z = q; q += 8 * BT;
-    W.V = q; q += 8 * BT;
-    W.C = q; q += NC + 2;
-    W.H = q; q += NC;
-    W.S = q; q += NC;
-    W.NET = q; q += L.nr;
-    W.X = q; q += BT;
-    W.red = q; q += 2 * (BT / 32);
-    W.slot = q; q += 4;
-    W.PIV = (int*)q;
-    W.ival = W.PIV + BT;
-    W.PERM = W.ival + BT / 32 + 1;
-  }
+  BlockShared W = carve_block<BT>((double*)bsm, L);
   const MechView M{(const double*)mech_gmem, (const int*)(mech_gmem + (size_t)L.n_double * sizeof(double))};
   for (long cell = blockIdx.x; cell < ncells; cell += gridDim.x) {
     __syncthreads();
