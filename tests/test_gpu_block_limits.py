@@ -8,8 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 def _most_reactions(nc, bt):
-    """(17 bt + 3 nc + nr + bt / 32 + 5) doubles, 2 bt + bt / 32 + 1 ints, 64 + 4 bytes, in 227 KB."""
-    return (227 * 1024 - 68 - 4 * (2 * bt + bt // 32 + 1)) // 8 - (17 * bt + 3 * nc + bt // 32 + 5)
+    """(17 bt + 3 nc + nr + bt / 32 + 5) doubles, 2 bt + bt / 32 + 1 ints, 64 + 16 bytes, in 227 KB."""
+    return (227 * 1024 - 80 - 4 * (2 * bt + bt // 32 + 1)) // 8 - (17 * bt + 3 * nc + bt // 32 + 5)
 
 
 def _mechanism(nc, nr):
