@@ -270,9 +270,10 @@ int lsg_ctx_kernel_times(lsg_ctx* ctx, double* ms, long long* launches, int nkin
  * lanes, plain warp kernel, persistent lane kernel, resident kernel 16 lanes,
  * resident kernel 32 lanes (0 for a candidate not tried).  A tuned context's
  * calls run either kernel of the batched form as LSG_TILE_LANE does: they wait
- * for the step, and calls smaller than the trial that the rounds won may run
- * the resident kernel, with the same results.  With LSG_JACOBIAN_ANALYTIC
- * only the rounds are tried, which honour it.  For mechanisms above 31 species with
+ * for the step, and calls smaller than a trial that the rounds won, or more than
+ * twice as large as one that the resident kernel won, run the kernel that
+ * LSG_TILE_LANE takes, with the same results.  With LSG_JACOBIAN_ANALYTIC only
+ * the rounds are tried, which honour it.  For mechanisms above 31 species with
  * LSG_PRECISION_MIXED the candidates are the block form with FP64 LU factors
  * (rates[0]) and with the tensor-core inverse (rates[1]), timed on one wave of
  * the FP64 form's blocks (at least 256 cells); tile is then LSG_TILE_BLOCK and

@@ -259,14 +259,15 @@ enum : int { kTunedRounds = 1, kTunedResident = 2 };
 // Lanes a cell of the batched form: the autotuner's, else 0 (by the number of components).
 int tuned_width(const lsg_ctx* c) { return c->tuned && c->tuned_tile == LSG_TILE_LANE ? c->tuned_w : 0; }
 
-// Whether the batched form's resident kernel takes a call: by the rule on sizes, unless the autotuner found the
-// resident kernel the faster (which it then is for smaller calls too), or the rounds for a call no larger than this one.
+// Whether the batched form's resident kernel takes a call: by the rule on sizes, or as the autotuner found on its trial
+// where that speaks for this call (large calls favour the rounds, small ones the resident kernel).
 bool takes_resident(const lsg_ctx* c, const StepOptions& so, long ncells) {
   if (c->tuned && c->tuned_tile == LSG_TILE_LANE) {
-    if (c->tuned_kernel == kTunedResident) return true;
-    if (ncells >= c->tuned_cells) return false;
+    if (c->tuned_kernel == kTunedResident && ncells <= 2 * c->tuned_cells) return true;
+    if (c->tuned_kernel == kTunedRounds && ncells >= c->tuned_cells) return false;
   }
-  return resident_applies(c->mech->host.layout, so, ncells, tuned_width(c), c->sm_count);
+  return resident_applies(c->mech->host.layout, so, c->opt.precision == LSG_PRECISION_FP64, ncells, tuned_width(c),
+                          c->sm_count);
 }
 
 int ensure_rounds(lsg_ctx* c, long n, bool lu64) {
@@ -431,7 +432,7 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
     c->tuned_tile = cd.tile;
     c->tuned_w = cd.w;
     c->tuned_kernel = cd.kernel;
-    c->tuned_cells = 0;
+    c->tuned_cells = cd.kernel == kTunedResident ? m : 0;   // this kernel, whatever the rule says
     float ms = 0.f;
     bool fits = true;
     for (int rep = 0; rep < 2 && fits; ++rep) {   // a 1024-cell run pays the one-time set-up, then the timed run
@@ -572,16 +573,21 @@ int launch_tile(lsg_ctx* c, const StepArgs& a, cudaStream_t s, int tile) {
   if (tile == LSG_TILE_LANE) {
     const bool lu64 = c->opt.precision == LSG_PRECISION_FP64;
     if (!sm_count(c)) return LSG_ERR_CUDA;
-    if (takes_resident(c, so, a.ncells)) {
-      const int r = launch_resident(c, a, so, tuned_width(c), s);
+    bool resident = takes_resident(c, so, a.ncells);
+    int r = resident ? LSG_OK : ensure_rounds(c, a.ncells, lu64);
+    if (r == LSG_ERR_NOMEM && so.jacobian == LSG_JACOBIAN_FD && resident_fits(L, tuned_width(c))) {
+      resident = true;   // no memory for the cells' records: the same results without them
+      r = LSG_OK;
+    }
+    if (r != LSG_OK) return r;
+    if (resident) {
+      r = launch_resident(c, a, so, tuned_width(c), s);
       if (r != LSG_OK) return r;
       // as with the round scheme, the call returns when the step is done
       if (cudaStreamSynchronize(s) != cudaSuccess) return LSG_ERR_CUDA;
       c->timer.collect();
       return LSG_OK;
     }
-    const int r = ensure_rounds(c, a.ncells, lu64);
-    if (r != LSG_OK) return r;
     const long max_rounds = 4L * (long)c->opt.max_steps * (L.nc + 9) + 64;
     const cudaError_t e = launch_rounds(c->rplan, L, c->mech->d_buf, so, a, c->rstate, c->rcap, c->nact_host,
                                         max_rounds, c->d_err, s, &c->launches, &c->timer);

@@ -165,7 +165,7 @@ cudaError_t launch_group(const MechLayout& L, const unsigned char* mech_gmem, co
                          bool lu64, int width, int* queue, int sm_count, cudaStream_t stream);
 // a block's shared memory holds at least one warp's cells, `width` lanes each (0: as launch_group)
 bool resident_fits(const MechLayout& L, int width = 0);
-bool resident_applies(const MechLayout& L, const StepOptions& o, long ncells, int width, int sm_count);
+bool resident_applies(const MechLayout& L, const StepOptions& o, bool lu64, long ncells, int width, int sm_count);
 
 // Jacobians with analytic species columns (lsg_rounds.cu), up to 31 species; J [ncells][n][n] row-major
 cudaError_t launch_jacobian(const MechLayout& L, const unsigned char* mech_gmem, long ncells, const double* y, long ld,

@@ -2354,17 +2354,29 @@ cudaError_t launch_rounds(const RoundsPlan& P, const MechLayout& L, const unsign
 }
 
 
-// Whether the resident form takes a call of the batched form.  It runs the solver of the round scheme bit for bit,
-// with forward differences only.  It was the faster of the two at every size where a block holds many cells
-// (H2/CO, 28 cells a block: 67 cells 7.2 against 63 ms, 20,011 cells 42 against 116 ms, 1,048,576 uneven cells 641
-// against 670 ms; CH4, 10 cells a block: 4,096 cells 105 against 672 ms, 65,536 cells 963 against 1,273 ms); with
-// few cells a block (many species or reactions) its time grows in proportion while the round scheme's floor, a
-// few hundred rounds of four launches, stays, so the round scheme takes large calls there.
-bool resident_applies(const MechLayout& L, const StepOptions& o, long ncells, int width, int sm_count) {
-  if (L.nc + 1 > 32 || o.jacobian != 0) return false;
-  if (width == 0) width = L.nc + 1 <= 16 ? 16 : 32;
+// Whether the resident form takes a call of the batched form.  It runs the solver of the round scheme bit for bit, with
+// forward differences only.  The rounds have a floor, some hundreds of rounds of four launches, which the resident form
+// beats at every small size; on large calls the cost of a further cell decides, and there the rounds are a little
+// cheaper.  So the rule is a number of cells for each that a block holds.  Measured on both sides, ms, resident against
+// rounds, cells of like stiffness (mixtures) unless said:
+//   few reactions for the components, FP32 factors: H2/CO, 28 cells a block, 65,536 120 against 175, 262,144 465 against
+//   521, 1,048,576 1,842 against 1,829; uneven cells 131,072 81 against 94, 524,288 317 against 311, 1,048,576 632
+//   against 596; 16 species, 16 cells a block, 131,072 419 against 453, 262,144 835 against 833, 524,288 1,660 against
+//   1,570; 28 species, 9 cells, 131,072 771 against 816, 262,144 1,540 against 1,543;
+//   FP64 factors, whose elimination costs the resident form more: H2/CO uneven 131,072 90 against 96, 524,288 353 against
+//   320; 16 species 65,536 201 against 231, 131,072 398 against 389;
+//   many reactions, whose rates wait while a block has fewer cells than its 32 evaluations: CH4, 10 cells, 155 reactions,
+//   32,768 486 against 616, 65,536 945 against 890, 131,072 1,864 against 1,456, but a flame's cells, for which the
+//   floor is high, 80,000 1,358 against 2,994, 160,000 2,591 against 3,731, 320,000 5,003 against 5,209: the line is
+//   between the two; FP64 factors alike;
+//   7 cells a block: 32,768 242 against 298, not measured above.
+bool resident_applies(const MechLayout& L, const StepOptions& o, bool lu64, long ncells, int width, int sm_count) {
+  const int n = L.nc + 1;
+  if (n > 32 || o.jacobian != 0) return false;
+  if (width == 0) width = n <= 16 ? 16 : 32;
   const int teams = team_count(L, width);
-  return teams >= 8 || ncells <= (long)sm_count * teams * 32;
+  const long most = teams < 8 ? 32 : L.nr > 3 * n ? 64 : lu64 ? 48 : 128;   // cells for each that a block holds
+  return ncells <= (long)sm_count * teams * most;
 }
 
 bool resident_fits(const MechLayout& L, int width) {

@@ -101,3 +101,38 @@ def test_batch_size_does_not_show(cuda, precision):
     part, ran = _step(data, A, np.ascontiguousarray(Y[:, :N]), T[:N], dt[:N], False, precision, 0)
     assert ran == {"group"}
     _same({k: np.ascontiguousarray(v[:N] if k == "counters" else v[..., :N]) for k, v in whole.items()}, part)
+
+
+@pytest.mark.parametrize("name,precision,line", [("ch4", 1, 10 * 64), ("ch4", 0, 10 * 64), ("h2co+2", 1, 16 * 128),
+                                                 ("h2co+2", 0, 16 * 48), ("h2co", 1, 28 * 128), ("h2co", 0, 28 * 48),
+                                                 ("h2co+17", 1, 7 * 32)])
+def test_large_calls_run_the_faster_kernel(cuda, name, precision, line):
+    """The resident kernel up to `line` cells an SM (the cells that fit a block, so many times over), the rounds above; the
+    cells are below tmin_chem, so that only the choice is run."""
+    import torch
+    data, species, A = _mechanism(name)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    sizes = [sms * line, sms * line + 1]
+    Y = np.full((len(species), sizes[-1]), 1.0)
+    out = []
+    for n, resident in zip(sizes, (True, False)):
+        o, ran = _step(data, A, np.ascontiguousarray(Y[:, :n]), np.full(n, 290.0), np.full(n, 1e-6), False, precision, 0)
+        assert (ran == {"group"}) == resident and ("init" in ran) != resident
+        out.append(o)
+    np.testing.assert_array_equal(out[0]["Y"], np.full((len(species), sizes[0]), 1.0 / len(species)))
+    _same({k: np.ascontiguousarray(v[:sizes[0]] if k == "counters" else v[..., :sizes[0]]) for k, v in out[1].items()},
+          out[0])
+
+
+def test_call_too_large_for_the_rounds(cuda, h2co):
+    """25 million cells: the rounds' records would take some 200 GB, so the resident kernel, which needs none, runs."""
+    import torch
+    from laminarsmoke_b200 import lsg
+    n = 25000000
+    ctx = lsg.ReactionStep(lsg.Mechanism(h2co[0]), tile=lsg.LSG_TILE_LANE, precision=1, tmin_chem=300.0)
+    Y = torch.full((14, n), 2.0, dtype=torch.float64, device=cuda)
+    T = torch.full((n,), 290.0, dtype=torch.float64, device=cuda)
+    ctx.step_device(Y, T, 1e-6)
+    torch.cuda.synchronize()
+    ctx.check()
+    assert bool((Y == 1.0 / 14.0).all())
