@@ -35,11 +35,21 @@ template <bool kStaged>
 __device__ __forceinline__ int warp_wofs(const MechLayout& L, int ws_doubles) {
   return (kStaged ? (int)(staged_bytes(L, L.warp_int) / 8u) : 0) + (int)(threadIdx.x >> 5) * ws_doubles;
 }
-// The warp's next cell: a block owns every gridDim-th cell, its warps take them in turn.
+// The warp's next cell: a block owns one cell of every gridDim in a row, its warps take them in turn.  Which one of the
+// row changes from row to row without a pattern, for the cells' cost has one: with the same place in every row, a mesh
+// whose lines are a multiple of gridDim long put the hot columns on a few blocks (296 x 40 H2/CO cells, ten hot columns,
+// 26.0 ms then, 10.2 now, 8.8 for the same cells shuffled).  A counter in global memory would do it too, but calls on
+// several streams, captured ones among them, could not share one.
 __device__ __forceinline__ long warp_cell() {
   int k = 0;
   if ((threadIdx.x & 31) == 0) k = atomicAdd(&warp_next(), 1);
-  return (long)blockIdx.x + (long)gridDim.x * __shfl_sync(kFull, k, 0);
+  k = __shfl_sync(kFull, k, 0);
+  unsigned h = (unsigned)k * 0x9e3779b9u;   // bits of k mixed; 0 for the first row
+  h = (h ^ (h >> 15)) * 0x2c1b3c6du;
+  h ^= h >> 13;
+  unsigned b = blockIdx.x + __umulhi(h, gridDim.x);
+  if (b >= gridDim.x) b -= gridDim.x;
+  return (long)gridDim.x * k + b;
 }
 }  // namespace
 
