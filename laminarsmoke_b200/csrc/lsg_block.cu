@@ -77,14 +77,6 @@ __device__ __forceinline__ double div0(double num, double den) {
   return z ? num * q : q;
 }
 
-// Value of thread src in every thread.
-__device__ __forceinline__ double bcast(double v, int src, double* slot) {
-  __syncthreads();
-  if ((int)threadIdx.x == src) *slot = v;
-  __syncthreads();
-  return *slot;
-}
-
 // Per-block shared work space.
 struct BlockShared {
   double* Z;     // [8][BT]
@@ -95,7 +87,7 @@ struct BlockShared {
   double* NET;   // [NR] net rates
   double* X;     // [BT] solve vector
   double* red;   // [2 BT/32]: bsum's partials
-  double* slot;  // [4]: broadcast, cached T, QR, pivot value
+  double* slot;  // [4]: the evaluation's T, the T of the kinetic constants, QR
   int* PIV;      // [BT]
   int* ival;     // [BT/32 + 1] pivot search scratch
   int* PERM;     // [BT] the factorisation's row interchanges composed: row i of P b is b[PERM[i]]

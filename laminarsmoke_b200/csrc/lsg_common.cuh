@@ -24,14 +24,6 @@ enum : int {
   kErrTensorCoreWait = 8,   // a tensor-core MMA did not report completion within the wait limit
 };
 
-// Sum of v over lanes 0..n-1, added strictly in lane order (the reference's
-// sequential loops).  Every lane receives the result.
-__device__ __forceinline__ double seq_sum(double v, int n) {
-  double s = 0.;
-  for (int i = 0; i < n; ++i) s += __shfl_sync(kFull, v, i);
-  return s;
-}
-
 // Rate constant of a pressure-logarithmic (PLOG) reaction at T and P
 // (PressureLogarithmicRateExpression::KineticConstant,
 // PressureLogarithmicRateExpression.hpp:104-119): the first or last point

@@ -253,7 +253,7 @@ __device__ __forceinline__ int eliminate_panel(float (&a)[kPanel], bool& pivoted
 __device__ __noinline__ bool gj_inverse(const double* __restrict__ J, int n, double hr0, const Smem& S,
                                         uint32_t tmem, uint32_t* phase) {
   const int tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
+  const int warp = tid >> 5;
   const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
   // ---- [G | I] into TMEM, row tid ----
   const double* const Jr = J + (tid < n ? tid : 0);

@@ -455,21 +455,18 @@ __device__ __noinline__ double rhs_slots(const Eval ev, bool live, double P0, in
 
 // G^-1, G = I - hr0 J, by Gauss-Jordan elimination in place with the pivots and the operations of gj_inverse:
 // its right half [I] only ever holds non-trivial entries in the columns already eliminated on the left, so
-// those columns of M hold them.  X receives G^-1 (FP64 words, rows of ld); M, the working matrix in the
-// precision LUT, is X itself (LUT double) or the upper half of X's memory (float), from which the rows move
-// down in order.  scr: n words for the pivot row, n ints for the interchanges.  The whole warp calls it; a
+// those columns hold them.  X receives G^-1 (rows of ld) and is the working matrix.  scr: n words for the pivot row, n
+// ints for the interchanges.  The whole warp calls it; a
 // team with on false passes through without a store.
-template <typename LUT, int W>
+template <int W>
 __device__ __noinline__ void gj_team(int oj, int ox, int osc, double hr0, int n, int lane, bool on) {
   const double* J = team_smem + oj;
   double* X = team_smem + ox;
-  double* scr = team_smem + osc;
+  double* K = team_smem + osc;
   const int ld = row_ld(n);
-  LUT* M = sizeof(LUT) == 4 ? (LUT*)X + n * ld : (LUT*)X;
-  LUT* K = (LUT*)scr;
-  int* perm = (int*)(scr + n);
+  int* perm = (int*)(K + n);
   const bool al = on && lane < n;
-  LUT* Mi = M + (lane < n ? lane : 0) * ld;
+  double* Xi = X + (lane < n ? lane : 0) * ld;
   __syncwarp();
   if (al) {
     const double* Ji = J + lane * ld;
@@ -477,30 +474,30 @@ __device__ __noinline__ void gj_team(int oj, int ox, int osc, double hr0, int n,
     for (int j = 0; j < n; ++j) {
       double g = -hr0 * Ji[j];
       if (j == lane) g += 1.;
-      Mi[j] = (LUT)g;
+      Xi[j] = g;
     }
     perm[lane] = lane;
   }
   __syncwarp();
 #pragma unroll 1
   for (int k = 0; k < n; ++k) {
-    LUT vv = (lane >= k && lane < n) ? (LUT)fabs((double)Mi[k]) : (LUT)-1;
+    double vv = (lane >= k && lane < n) ? fabs(Xi[k]) : -1.;
     int r = lane;
 #pragma unroll
     for (int off = W / 2; off > 0; off >>= 1) {
-      const LUT ov = __shfl_xor_sync(kFull, vv, off, W);
+      const double ov = __shfl_xor_sync(kFull, vv, off, W);
       const int orr = __shfl_xor_sync(kFull, r, off, W);
       if (ov > vv || (ov == vv && orr < r)) { vv = ov; r = orr; }
     }
     r = __shfl_sync(kFull, r, 0, W);
     if (r < k || r >= n) r = k;   // a NaN column cannot send the pivot outside rows k..n-1
-    const LUT pv = M[r * ld + k];
-    const LUT ipv = (pv != (LUT)0) ? (LUT)1 / pv : (LUT)0;
+    const double pv = X[r * ld + k];
+    const double ipv = pv != 0. ? 1. / pv : 0.;
     __syncwarp();                 // every lane has the pivot before its row moves
     if (al) {
-      const LUT ak = M[k * ld + lane], ar = M[r * ld + lane];
+      const double ak = X[k * ld + lane], ar = X[r * ld + lane];
       K[lane] = lane == k ? ipv : ar * ipv;
-      if (r != k) M[r * ld + lane] = ak;
+      if (r != k) X[r * ld + lane] = ak;
       if (lane == 0) {
         const int t = perm[k];
         perm[k] = perm[r];
@@ -509,36 +506,36 @@ __device__ __noinline__ void gj_team(int oj, int ox, int osc, double hr0, int n,
     }
     __syncwarp();
     if (al && lane != k) {
-      const LUT fct = Mi[k];
-      Mi[k] = (LUT)0;
+      const double fct = Xi[k];
+      Xi[k] = 0.;
       int j = 0;
 #pragma unroll 1
       for (; j + 4 <= n; j += 4) {
-        const LUT a0 = Mi[j], a1 = Mi[j + 1], a2 = Mi[j + 2], a3 = Mi[j + 3];
-        const LUT k0 = K[j], k1 = K[j + 1], k2 = K[j + 2], k3 = K[j + 3];
-        Mi[j] = a0 - fct * k0;
-        Mi[j + 1] = a1 - fct * k1;
-        Mi[j + 2] = a2 - fct * k2;
-        Mi[j + 3] = a3 - fct * k3;
+        const double a0 = Xi[j], a1 = Xi[j + 1], a2 = Xi[j + 2], a3 = Xi[j + 3];
+        const double k0 = K[j], k1 = K[j + 1], k2 = K[j + 2], k3 = K[j + 3];
+        Xi[j] = a0 - fct * k0;
+        Xi[j + 1] = a1 - fct * k1;
+        Xi[j + 2] = a2 - fct * k2;
+        Xi[j + 3] = a3 - fct * k3;
       }
 #pragma unroll 1
-      for (; j < n; ++j) Mi[j] = Mi[j] - fct * K[j];
+      for (; j < n; ++j) Xi[j] = Xi[j] - fct * K[j];
     }
     __syncwarp();
-    if (al) M[k * ld + lane] = K[lane];
+    if (al) X[k * ld + lane] = K[lane];
     __syncwarp();
   }
   const int pc = al ? perm[lane] : 0;
 #pragma unroll 1
   for (int i = 0; i < n; ++i) {
-    const double g = al ? (double)M[i * ld + lane] : 0.;
+    const double g = al ? X[i * ld + lane] : 0.;
     __syncwarp();
     if (al) X[i * ld + pc] = g;
     __syncwarp();
   }
 }
 
-// gj_team in FP32 with the lane's row in registers, padded with zero columns to W: the column being eliminated is
+// gj_team's FP32 counterpart with the lane's row in registers, padded with zero columns to W: the column being eliminated is
 // always a[0] and the row moves down by one with each pivot, so that every index is static; rows stay in their
 // lanes and `pos` holds their place in the pivoted order (the interchanges move places, not data).
 template <int W>
@@ -781,7 +778,7 @@ __device__ __noinline__ int advance_team(int ro, int cell, int lane, unsigned gm
     }
     if (any(factor)) {
       if constexpr (sizeof(LUT) == 4) gj_reg<W>(ro + TL.oj, ro + TL.ox, hr0f, n, lane, gm, factor);
-      else gj_team<LUT, W>(ro + TL.oj, ro + TL.ox, sc, hr0f, n, lane, factor);
+      else gj_team<W>(ro + TL.oj, ro + TL.ox, sc, hr0f, n, lane, factor);
       if (factor) {
         const int c = RI[I_CNT0 + CNT_FACT], cj = RI[I_CNT0 + CNT_JAC];
         __syncwarp(gm);

@@ -4,8 +4,8 @@
 // fraction l, lane NC owns T); reaction-parallel work (rate constants,
 // products of concentrations) is spread over the 32 lanes.  Every quantity the
 // reference accumulates sequentially (mixture sums, WRMS norms, L1 norms,
-// formation rates, reaction enthalpies) is accumulated in the same order here
-// (seq_sum), so with FMA contraction disabled this path reproduces the CPU
+// formation rates, reaction enthalpies) is accumulated in the same order here,
+// from shared memory (sum_shared), so with FMA contraction disabled this path reproduces the CPU
 // algorithm operation for operation; the remaining differences come from the
 // device exp/log/pow, which agree with the host's to about one ulp.
 //
