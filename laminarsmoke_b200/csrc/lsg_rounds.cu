@@ -1368,8 +1368,11 @@ __device__ __noinline__ void steady_sparse_diagonal(const MechLayout* __restrict
 // zero) and the temperature entry by the forward difference of the dense path (with energyEquation on,
 // else zero).  A block takes 128 cells' source terms, their source terms at the incremented temperature or
 // their diagonal (kind 0, 1, 2): a thread's dependent chain bounds the kernel, and the three are independent,
-// so apart they take less time where the SMs are not full (CH4, 1000 cells: 996 to 693 us) and fill the last wave
-// better where they are (H2/CO, 80 000 cells: 572 to 529 us).  yb, s0, sp: scratch [n][ncells]; kind 1 keeps its state in Sexp.
+// so apart they take less time where the SMs are not full (CH4, 1000 cells: 1,251 us in one kernel with the reactions'
+// lists, 680 now) and fill the last wave better where they are (H2/CO, 80 000 cells: 740 and 515 us).  y0, s0, y1:
+// scratch [n][ncells], the states of kinds 0 and 1 and the source terms of kind 0; the one source term of kind 1 that is
+// used, the heat release, goes to y0's temperature row, which is not (the others to the same place before it).  Sexp is
+// written by the combination alone, so that it may take the place of the state.
 __device__ __forceinline__ double steady_t_increment(double yk) {   // linearModel.H:195-230, for the T entry
   const double ew = 1. / (1.e-12 + 1.e-7 * fabs(yk));
   double hJ = sqrt(kMachEpsDouble) * fabs(fmax(yk, 1. / ew));
@@ -1380,8 +1383,8 @@ __device__ __forceinline__ double steady_t_increment(double yk) {   // linearMod
 __global__ void __launch_bounds__(kRT, 4) steady_sources_sparse_kernel(
     MechLayout Lp, const unsigned char* __restrict__ mech_gmem, long ncells, const double* __restrict__ Y,
     const double* __restrict__ T, long ld, const double* __restrict__ pc, double p_scalar, int species, int energy,
-    double* __restrict__ yb, double* __restrict__ s0, double* __restrict__ sp, double* __restrict__ Simp,
-    double* __restrict__ Sexp, long lds, int* err) {
+    double* __restrict__ y0, double* __restrict__ s0, double* __restrict__ y1, double* __restrict__ Simp, long lds,
+    int* err) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ MechLayout sL;
@@ -1405,20 +1408,20 @@ __global__ void __launch_bounds__(kRT, 4) steady_sources_sparse_kernel(
       continue;
     }
     if (kind == 1 && !energy) continue;
-    double* const y = (kind ? Sexp : yb) + c;
-    double* const f = (kind ? sp : s0) + c;
-    const long ys = kind ? lds : ncells;
-    for (int i = 0; i < NC; ++i) y[(long)i * ys] = fmax(Y[(long)i * ld + c], 0.);
-    y[(long)NC * ys] = T[c];
-    const double q = rhs_cell<true>(&sL, Md, Mi, scratch, y, ys, kind ? NC : -1, T[c] + steady_t_increment(T[c]), f,
-                                    ncells, P0, 1, 0.);
-    f[(long)NC * ncells] = q;
+    double* const y = (kind ? y1 : y0) + c;
+    double* const f = kind ? y0 + (long)NC * ncells + c : s0 + c;
+    const long fs = kind ? 0 : ncells;
+    for (int i = 0; i < NC; ++i) y[(long)i * ncells] = fmax(Y[(long)i * ld + c], 0.);
+    const double Tc = kind ? T[c] + steady_t_increment(T[c]) : T[c];
+    const double q = rhs_cell<true>(&sL, Md, Mi, scratch, y, ncells, NC, Tc, f, fs, P0, 1, 0.);
+    f[(long)NC * fs] = q;
   }
 }
-// The temperature entry from kinds 0 and 1, and the explicit part of component blockIdx.y.
+// The temperature entry from kinds 0 and 1 (q1: the heat release of kind 1), and the explicit part of component
+// blockIdx.y.
 __global__ void __launch_bounds__(256) steady_sources_combine_kernel(
     int NC, long ncells, const double* __restrict__ Y, const double* __restrict__ T, long ld, int energy,
-    const double* __restrict__ s0, const double* __restrict__ sp, double* __restrict__ Simp, double* __restrict__ Sexp,
+    const double* __restrict__ s0, const double* __restrict__ q1, double* __restrict__ Simp, double* __restrict__ Sexp,
     long lds) {
   const int k = blockIdx.y;
   for (long c = (long)blockIdx.x * 256 + threadIdx.x; c < ncells; c += (long)gridDim.x * 256) {
@@ -1429,7 +1432,7 @@ __global__ void __launch_bounds__(256) steady_sources_combine_kernel(
       yk = Y[(long)k * ld + c];
     } else {
       yk = T[c];
-      J = energy ? (sp[(long)k * ncells + c] - s) * (1. / steady_t_increment(yk)) : 0.;
+      J = energy ? (q1[c] - s) * (1. / steady_t_increment(yk)) : 0.;
       Simp[(long)k * lds + c] = J;
     }
     Sexp[(long)k * lds + c] = s - J * yk;
@@ -2249,12 +2252,12 @@ cudaError_t launch_steady_sources_sparse(const MechLayout& L, const unsigned cha
   const long n = L.nc + 1;
   steady_sources_sparse_kernel<<<(unsigned)(want < cap ? want : cap), kRT, smem, stream>>>(
       L, mech_gmem, ncells, Y, T, ld, p, p_scalar, species, energy, scratch, scratch + n * ncells,
-      scratch + 2 * n * ncells, Simp, Sexp, lds, err);
+      scratch + 2 * n * ncells, Simp, lds, err);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const long cells256 = (ncells + 255) / 256;
   const dim3 grid((unsigned)(cells256 < 4096 ? cells256 : 4096), (unsigned)n);
   steady_sources_combine_kernel<<<grid, 256, 0, stream>>>(L.nc, ncells, Y, T, ld, energy, scratch + n * ncells,
-                                                          scratch + 2 * n * ncells, Simp, Sexp, lds);
+                                                          scratch + L.nc * ncells, Simp, Sexp, lds);
   return cudaGetLastError();
 }
 

@@ -124,3 +124,27 @@ def test_gpu_steady_sources_sparse(cuda, name, species, energy):
         tolT = 1e-6 * abs(ri[-1]) + 64 * 2.220446049250313e-16 * abs(s0[-1]) / dT
         assert abs(si[c, -1] - ri[-1]) <= tolT, (c, si[c, -1], ri[-1])
         np.testing.assert_allclose(se[c] + si[c] * y, s0, rtol=1e-10, atol=1e-12 * np.abs(s0).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["h2co", "ch4"])
+def test_gpu_explicit_part_in_the_place_of_the_state(cuda, name):
+    """S_explicit given the memory of a stacked state (mass fractions, then the temperature): the same bits as in an
+    array of its own, negative mass fractions included, whose explicit part uses them unclipped."""
+    import torch
+    from laminarsmoke_b200 import lsg, mech
+    data, sp = mech.load(name)
+    nc, n = len(sp), 700
+    rng = np.random.default_rng(67)
+    Y = 10.0 ** rng.uniform(-9, 0, (nc, n))
+    Y[rng.random((nc, n)) < 0.1] = -1e-3
+    y = torch.tensor(np.concatenate([Y, rng.uniform(800.0, 2400.0, (1, n))]), device=cuda)
+    ctx = lsg.ReactionStep(lsg.Mechanism(data))
+    Si, Se = torch.zeros_like(y), torch.zeros_like(y)
+    ctx.steady_sources_sparse_device(y[:nc].clone(), y[nc].clone(), Si, Se)
+    state, Si2 = y.clone(), torch.zeros_like(y)
+    ctx.steady_sources_sparse_device(state[:nc], state[nc], Si2, state)
+    torch.cuda.synchronize()
+    ctx.check()
+    np.testing.assert_array_equal(Si2.cpu().numpy(), Si.cpu().numpy())
+    np.testing.assert_array_equal(state.cpu().numpy(), Se.cpu().numpy())
