@@ -172,12 +172,12 @@ def parse():
     ap.add_argument("--cpu-sample", type=int, default=0,
                     help="cells of the CPU baseline sample (0: sized for about 10 s of CPU work)")
     ap.add_argument("--tile", choices=("auto", "lane", "persistent", "group"), default="auto",
-                    help="batched form: autotuned (the first warm-up step times the candidate forms), round "
-                         "scheme (lane) or persistent lane kernel")
+                    help="batched form: autotuned (the first warm-up step times the candidate forms), by the rule on "
+                         "sizes (lane), its resident kernel (group) or the persistent lane kernel")
     ap.add_argument("--factors", choices=("fp32", "fp64"), default="fp32",
                     help="batched form: precision of the LU factors")
     ap.add_argument("--plain-steps", type=int, default=3,
-                    help="timed steps of the plain FP64 form (it is ~6x slower; 0 skips it)")
+                    help="timed steps of the plain FP64 form (it is ~3x slower; 0 skips it)")
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--plain-cells", type=int, default=0,
                     help="large-mechanism workloads: the FP64 arm runs on an evenly strided sample of this many "

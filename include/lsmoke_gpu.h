@@ -50,8 +50,8 @@ extern "C" {
 #define LSG_TILE_AUTO 0        /* FP64 -> warp per cell; MIXED -> the batched form (up to 31 species) */
 #define LSG_TILE_WARP 1        /* one warp per cell, the reference's operation order (FP64 only) */
 #define LSG_TILE_LANE 2        /* the batched form: cells resident in shared memory from start to finish, many to a
-                                  block, or (few cells a block, analytic Jacobian) rounds of RHS / solver kernels over
-                                  the live cells; the same results either way */
+                                  block, or (large calls, analytic Jacobian) rounds of RHS / solver kernels over the
+                                  live cells; with the same Jacobian the same results either way */
 #define LSG_TILE_PERSISTENT 3  /* one thread per cell, one persistent kernel + device work queue */
 #define LSG_TILE_BLOCK 4       /* one thread block per cell (any size up to 511 species) */
 #define LSG_TILE_GROUP 5       /* the batched form's resident kernel, called asynchronously (up to 31 species); where
@@ -275,8 +275,8 @@ int lsg_ctx_kernel_times(lsg_ctx* ctx, double* ms, long long* launches, int nkin
  * LSG_TILE_LANE takes, with the same results.  With LSG_JACOBIAN_ANALYTIC only
  * the rounds are tried, which honour it.  For mechanisms above 31 species with
  * LSG_PRECISION_MIXED the candidates are the block form with FP64 LU factors
- * (rates[0]) and with the tensor-core inverse (rates[1]), timed on one wave of
- * the FP64 form's blocks (at least 256 cells); tile is then LSG_TILE_BLOCK and
+ * (rates[0]) and with the tensor-core inverse (rates[1]), timed on the call's
+ * first cells, at most four for each SM (calls of at least 256 cells); tile is then LSG_TILE_BLOCK and
  * the variant 1 for the tensor-core inverse, 0 for the FP64 factors.  Returns
  * LSG_ERR_ARG when no tuning has run yet. */
 #define LSG_NTUNE_CANDIDATES 6

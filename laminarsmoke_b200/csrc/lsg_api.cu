@@ -476,8 +476,8 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
 
 // Autotuner for mechanisms above 31 species with mixed precision: the block form with the FP64 LU factors
 // (rates[0]) against the block form with the tensor-core inverse (rates[1]), each timed on (a copy of) the
-// first min(ncells, slots of the FP64 form) cells, one wave of the FP64 form.  The tensor-core form holds
-// more shared memory and TMEM per block, so it runs fewer blocks per SM where the FP64 form fits more;
+// first min(ncells, work spaces of the FP64 form) cells: up to four an SM up to 128 components, one above.  The FP64
+// form then runs one block per SM with its factors in shared memory, the tensor-core form two;
 // which is faster depends on how much of the step the factorisations are.  Keeps tile LSG_TILE_BLOCK with
 // width 1 (tensor-core inverse) or 0 (FP64 factors).
 int autotune_large(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {

@@ -2384,10 +2384,10 @@ cudaError_t block_plan(const MechLayout& L, int sm_count, bool tc, long* nblocks
 namespace {
 // Whether the FP64 form keeps a cell's factors in shared memory, one block of 256 threads an SM (more threads spill
 // their registers), instead of four blocks of 128 threads with the factors in the L2: whenever they fit, which leaves
-// the other form to more than some 7000 reactions.  Faster at every size and count measured (ms, before and after):
-// 45 components 22.0 and 11.4 at 96 cells, 42.5 and 35.4 at 592, 1986 and 1469 at 30 000; 121 components 18.3 and 6.2
-// at one cell, 88.9 and 60.9 at 592, 694 and 485 at 6000; 800 reactions and 121 components 811 and 357 at 96 cells,
-// 1798 and 1377 at 1200.
+// the other form to more than some 7000 reactions.  Faster at every size and count measured (ms, without and
+// with): 45 components 20.8 and 10.2 at 96 cells, 40.5 and 31.7 at 592, 1846 and 1321 at 30 000; 121 components 17.3 and
+// 5.7 at one cell, 89.0 and 56.6 at 592, 659 and 452 at 6000; 800 reactions and 121 components 651 and 293 at 96 cells,
+// 1797 and 1383 at 1200.
 constexpr size_t kSgSmem = 225 * 1024;   // of 227 KB: the rest for the static shared memory and the block's reserve
 bool shared_factors(const MechLayout& L) { return block_sg_bytes<256>(L) <= kSgSmem; }
 }  // namespace

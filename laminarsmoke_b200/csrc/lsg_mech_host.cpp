@@ -107,14 +107,14 @@ static void fit_range(const std::vector<const std::vector<double>*>& fits, doubl
   *lo = 1.;
   *hi = 0.;
   if (!within(mid, mid)) return;
-  double a = mid, b = mid;
-  double out = -750.;   // below ln of the smallest positive double
-  for (int i = 0; i < 64; ++i) {
+  double a = mid, b = mid;   // within; some twelve halvings on either side, for the range need not be sharp
+  double out = -750.;        // below ln of the smallest positive double
+  for (int i = 0; i < 12; ++i) {
     const double x = 0.5 * (a + out);
     (within(x, b) ? a : out) = x;
   }
-  out = 710.;           // above ln of the largest
-  for (int i = 0; i < 64; ++i) {
+  out = 710.;                // above ln of the largest
+  for (int i = 0; i < 12; ++i) {
     const double x = 0.5 * (b + out);
     (within(a, x) ? b : out) = x;
   }

@@ -29,16 +29,18 @@
 // ones read as warp-uniform 16-byte loads through L1, which the streamed rows
 // bypass.
 //
-// The kernel is bound by the FP64 pipe, not by HBM: nc (nc - 1) / 2 binary
-// fits, each an exponential, then nc^2 Wilke terms.  So the exponentials of the
+// What a cell costs is arithmetic, not HBM: nc (nc - 1) / 2 binary fits, each an
+// exponential, then nc^2 Wilke terms.  The FP64 pipe is 50 % busy; the rest are
+// dependent chains in the 8 to 24 warps of an SM and, in Wilke's loop, shared
+// memory (two work array entries and two table entries for every two pairs).  So the exponentials of the
 // fits are a range reduction and a Taylor polynomial inline (exp_fit: 20
 // instructions against some 60 of the library's), no pair divides (1 / D by the
 // negated fit, sqrt(eta) and its reciprocal by half the fit's exponent), and a
 // pair's Wilke terms use sqrt(phi) from the host.  Contraction is off: the sums
 // whose terms cancel (h, the Soret terms) round like the host arithmetic, the others are written
 // with fma.  1,048,576 H2/CO cells with
-// every field: 1,510 us before, 630 us now (FP64 pipe 50 % busy; the bytes alone:
-// 92 us); 39,999 CH4 cells: 245 us before, 127 us now.
+// every field: 1,510 us with divisions and the library's exponentials, 630 us now
+// (the bytes alone: 92 us); 39,999 CH4 cells: 245 and 127 us.
 #include "lsg_common.cuh"
 #include "lsg_kernels.h"
 

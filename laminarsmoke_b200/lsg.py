@@ -361,7 +361,7 @@ class ReactionStep:
     def step_sequence_graph(self, Y, T, dt: float, nsteps: int, p: float = 101325.0, t0: float = 0.0, Q=None,
                             status=None, stream=None) -> bool:
         """lsg_reaction_step_sequence_device: `nsteps` successive steps of the device-resident cells,
-        captured once into a CUDA graph by the library and replayed (the round scheme runs them one by
+        captured once into a CUDA graph by the library and replayed (the batched form runs them one by
         one).  Returns True when the graph ran."""
         _require_layout(Y, T, Q, status)
         nc, ld = Y.shape
@@ -513,6 +513,8 @@ class ReactionStep:
                "lsg_ctx_kernel_times")
         return {k: (ms[i], nl[i]) for i, k in enumerate(self.KERNEL_KINDS)}
 
+    # the batched form's rounds (LSG_TILE_LANE) and resident kernel (LSG_TILE_GROUP variants 4 and 2) with 16 and 32
+    # lanes per cell, and the forms between
     TUNE_CANDIDATES = ("rounds16", "rounds32", "plain_warp", "persistent", "group_4", "group_2")
     # mechanisms above 31 species, mixed precision: the block form's factorisation
     TUNE_CANDIDATES_LARGE = ("block_fp64_lu", "block_tc_inverse")
