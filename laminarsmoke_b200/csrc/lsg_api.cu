@@ -438,6 +438,9 @@ int autotune(lsg_ctx* c, const StepArgs& a, cudaStream_t s) {
     for (int rep = 0; rep < 2 && fits; ++rep) {   // a 1024-cell run pays the one-time set-up, then the timed run
       if (cudaMemcpyAsync(work, pristine, per * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
         c->timer.on = timing;
+        c->tuned = false;
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
         return LSG_ERR_CUDA;
       }
       StepArgs tr = t;
